@@ -866,14 +866,17 @@ static void sched_store_locked(const std::string &key, const std::string &val) {
   fclose(f);
 }
 
+// Raised when the step kernels change, so that a file's measurements of older ones are not used.
+#define KWB_SCHED_GEN 2
+
 static std::string sched_key(int device, const SimDev &h) {
   cudaDeviceProp prop;
   char name[256] = "unknown";
   if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) snprintf(name, sizeof(name), "%s/%d", prop.name, prop.multiProcessorCount);
   char buf[512];
   const char *eo = getenv("KWB_TUNE_ORDER");
-  snprintf(buf, sizeof(buf), "%.200s|v%d|nd%d|N%dx%dx%d|fast%d|plane%d|fuse%d|disp%d|fill%d|axi%d|rho%d|c%d|nl%d|ord%d",
-           name, KWB_VERSION, h.ndim, h.N[0], h.N[1], h.N[2], h.fast, h.plane, h.fuse_xeos, h.dispersion,
+  snprintf(buf, sizeof(buf), "%.200s|v%d.%d|nd%d|N%dx%dx%d|fast%d|plane%d|fuse%d|disp%d|fill%d|axi%d|rho%d|c%d|nl%d|ord%d",
+           name, KWB_VERSION, KWB_SCHED_GEN, h.ndim, h.N[0], h.N[1], h.N[2], h.fast, h.plane, h.fuse_xeos, h.dispersion,
            h.grid_fill, h.inv_r ? 1 : 0, h.rho0 ? 1 : 0, h.c0sq ? 1 : 0, (h.nonlinear && h.nlq) ? 2 : h.nonlinear,
            (eo && strcmp(eo, "1") == 0) ? 1 : 0);
   return buf;
@@ -1276,6 +1279,14 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
     h.gneg[a] = gn;
     h.pml_def[a] = pd;
     h.pml_sg_def[a] = psd;
+    if (h.fast && a < D && fast_size(n)) {
+      size_t bytes = 0;
+      CU(fast_image(n, nullptr, &bytes, tw, gp, gn, psd, pd, st));
+      float2 *img;
+      CU(M.alloc(&img, bytes / sizeof(float2)));
+      CU(fast_image(n, img, nullptr, tw, gp, gn, psd, pd, st));
+      h.img[a] = img;
+    }
   }
   if (P->axisymmetric) {
     // 1/r on the radial axis: r = |y_vec|, y_vec = ((0:Ny-1) - (Ny-1)/2) dy, r = 0 -> dy/2

@@ -162,6 +162,15 @@ cudaError_t fast_prime(int N) {
   cudaError_t e = prime_eos(N);
   return e != cudaSuccess ? e : prime_line(N);
 }
+cudaError_t fast_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                       const float *pml_sg, const float *pml, cudaStream_t st) {
+  if (fast_mixed_size(N)) return fast_mixed_image(N, img, bytes, tw, gpos, gneg, pml_sg, pml, st);
+  if (fast_mixed2_size(N)) return fast_mixed2_image(N, img, bytes, tw, gpos, gneg, pml_sg, pml, st);
+  if (fast_mixed3_size(N)) return fast_mixed3_image(N, img, bytes, tw, gpos, gneg, pml_sg, pml, st);
+  if (fast_mixed4_size(N)) return fast_mixed4_image(N, img, bytes, tw, gpos, gneg, pml_sg, pml, st);
+  if (fast_mixed5_size(N)) return fast_mixed5_image(N, img, bytes, tw, gpos, gneg, pml_sg, pml, st);
+  KWB_LINE_SWITCH(N, image_n, (img, bytes, tw, gpos, gneg, pml_sg, pml, st))
+}
 cudaError_t fast_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                            cudaStream_t st) {
   if (fast_mixed_size(h.N[axis])) return fast_mixed_line_pass(d_sim, h, axis, mode, s, st);

@@ -686,60 +686,63 @@ struct LineFFT4G {
   }
 };
 
-// Build the per-CTA tables: tw2 (and, for line passes, the gradient multipliers in register order).
-template <int E, int G>
-__device__ __forceinline__ void build_tables(float2 *tw2, float2 *gp2, float2 *gn2, const float2 *tw,
-                                             const float2 *gpos, const float2 *gneg) {
-  constexpr int RP = G + 1, J = E / G;
-  for (int e = threadIdx.x; e < E * G; e += blockDim.x) {
-    const int q = e / G, u = e - q * G;
-    tw2[q * RP + u] = tw[u * q];
-    if (gp2) {
-      const int k = u * J + q / G + E * (q % G);
-      gp2[q * RP + u] = gpos[k];
-      gn2[q * RP + u] = gneg[k];
-    }
-  }
-}
-
-// Line-pass tables for an FFT policy F: twiddles, then the gradient multipliers i k e^{+-ikd/2}/N
-// in register order [idx][t] (pitch G+1).
+// Table image of one axis for an FFT policy F, built once per simulation in the order the kernels
+// hold it in shared memory: the twiddles (F::TW), the gradient multipliers i k e^{+-ikd/2}/N in
+// register order [idx][t] (pitch G+1; staggered + then -), then the two PML deficits (staggered,
+// plain).  A CTA copies it with 16-byte asynchronous copies while its predecessor still runs; the
+// same tables gathered entry by entry, with their index arithmetic, took 1.5 us at the start of
+// each kernel (512^2, 128-thread CTAs) on the critical path of a small grid's step.
 template <class F>
-__device__ __forceinline__ void build_line_tables(float2 *tw, float2 *gp2, float2 *gn2, const float2 *g,
-                                                  const float2 *gpos, const float2 *gneg) {
-  F::build_tw(tw, g);
+__host__ __device__ constexpr int image_pairs() {
+  return F::TW + 2 * F::E * (F::G + 1);
+}
+template <class F>
+__host__ __device__ constexpr size_t image_bytes() {
+  return ((size_t)image_pairs<F>() * sizeof(float2) + 2 * (size_t)F::N * sizeof(float) + 15) & ~size_t(15);
+}
+// The part of it a line pass holds in shared memory: all of it up to N = 512; longer lines, whose
+// full-width tiles leave no room for the deficits, read them from global memory, one batch a pass.
+template <class F>
+__host__ __device__ constexpr bool image_pml() {
+  return F::N <= 512;
+}
+template <class F>
+__host__ __device__ constexpr size_t image_line_bytes() {
+  return image_pml<F>() ? image_bytes<F>() : ((size_t)image_pairs<F>() * sizeof(float2) + 15) & ~size_t(15);
+}
+// ... of its twiddles alone (the equation-of-state and spectrum passes)
+template <class F>
+__host__ __device__ constexpr size_t image_tw_bytes() {
+  return ((size_t)F::TW * sizeof(float2) + 15) & ~size_t(15);
+}
+template <class F>
+__global__ void __launch_bounds__(256)
+    k_build_image(float2 *img, const float2 *g, const float2 *gpos, const float2 *gneg, const float *pml_sg,
+                  const float *pml) {
+  F::build_tw(img, g);
   constexpr int RP = F::G + 1;
-  for (int e = threadIdx.x; e < F::E * F::G; e += blockDim.x) {
-    const int q = e / F::G, u = e - q * F::G;
-    const int k = F::k_of(u, q);
-    gp2[q * RP + u] = gpos[k];
-    gn2[q * RP + u] = gneg[k];
+  float2 *gp = img + F::TW, *gn = gp + F::E * RP;
+  for (int e = threadIdx.x; e < F::E * RP; e += blockDim.x) {
+    const int q = e / RP, u = e - q * RP;
+    const int k = u < F::G ? F::k_of(u, q) : 0;  // column G is padding
+    gp[e] = gpos[k];
+    gn[e] = gneg[k];
+  }
+  float *pm = reinterpret_cast<float *>(gn + F::E * RP);
+  for (int i = threadIdx.x; i < F::N; i += blockDim.x) {
+    pm[i] = pml_sg[i];
+    pm[F::N + i] = pml[i];
   }
 }
-// Register line pass: exchange buffers, twiddles and gradient tables, then the two staged operand
-// tiles, 128-byte aligned (destinations of tiled TMA copies).
+// Register line pass: exchange buffers and table image, then the two staged operand tiles,
+// 128-byte aligned (destinations of tiled TMA copies).
 template <class F>
 __host__ __device__ constexpr size_t pline_offset(int L) {
-  return (((size_t)L * F::LP + F::TW + 2 * (size_t)F::E * (F::G + 1)) * sizeof(float2) + 127) & ~size_t(127);
+  return ((size_t)L * F::LP * sizeof(float2) + image_line_bytes<F>() + 127) & ~size_t(127);
 }
 template <class F>
 __host__ __device__ constexpr size_t pline_smem(int L) {
   return pline_offset<F>(L) + 2 * (size_t)(2 * L) * F::N * sizeof(float);
-}
-
-template <int E, int G>
-__host__ __device__ constexpr size_t line_smem(int L) {
-  return ((size_t)L * (E * (G + 1) + 1) + 3 * (size_t)E * (G + 1)) * sizeof(float2);
-}
-// Line pass: the exchange buffers and tables, then two staged operand tiles (p and rho0) of
-// 2L real lines x N floats each, 16-byte aligned.
-template <int E, int G>
-__host__ __device__ constexpr size_t line_stage_offset(int L) {
-  return (line_smem<E, G>(L) + 15) & ~size_t(15);
-}
-template <int E, int G>
-__host__ __device__ constexpr size_t line_smem_staged(int L) {
-  return line_stage_offset<E, G>(L) + 2 * (size_t)(2 * L) * (E * G) * sizeof(float);
 }
 
 // 16-byte asynchronous global->shared copy; bytes beyond src_bytes are zero-filled.
@@ -750,6 +753,21 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// Copy `bytes` (a multiple of 16) of an axis's table image into shared memory, as one group.  The
+// copies allocate in L1 (.ca): the CTAs that follow on an SM take the image from there.
+__device__ __forceinline__ void stage_image(void *dst, const float2 *img, size_t bytes) {
+  for (unsigned c = threadIdx.x; c < (unsigned)(bytes / 16); c += blockDim.x)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(reinterpret_cast<char *>(dst) + 16 * c)),
+                 "l"(reinterpret_cast<const char *>(img) + 16 * c)
+                 : "memory");
+  cp_async_commit();
+}
+// Programmatic dependent launch (see KWB_STEP_KERNEL_PROLOGUE): a kernel may read what kernels
+// before its predecessor wrote without waiting, since its predecessor let it start only after its
+// own wait; what its predecessor wrote, only after pdl_wait().
+__device__ __forceinline__ void pdl_wait() { KWB_STEP_KERNEL_PROLOGUE(); }
 
 // Bulk (TMA) copies global -> shared completing on an mbarrier (no multicast).
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -820,6 +838,9 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   float2 *tw2 = sm + L * LP;
   float2 *gp2 = tw2 + F::TW;
   float2 *gn2 = gp2 + E * RP;
+  constexpr bool PML_S = image_pml<F>();
+  // staggered deficits, then plain
+  const float *pml_s = reinterpret_cast<const float *>(PML_S ? gn2 + E * RP : S.img[axis] + image_pairs<F>());
   // Contiguous tiles are 2L whole consecutive rows, so each field's tile is one block of
   // memory: one bulk (TMA) copy per field.  Strided tiles (2L columns of N rows) are boxes of
   // the field's tensor map: N / tile_box_rows tiled TMA copies per field.  Each field's copies
@@ -835,15 +856,15 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
 #pragma unroll
     for (int b = 0; b < 4; ++b) mbar_init(&tile_bar[b], 1);
   }
-  // the tables are written once at set-up: built before waiting on the previous kernel
-  build_line_tables<F>(tw2, gp2, gn2, S.tw[axis], S.gpos[axis], S.gneg[axis]);
+  // the table image is written once at set-up: copied before waiting on the previous kernel
+  stage_image(tw2, S.img[axis], image_line_bytes<F>());
   if (tma) __syncthreads();  // the mbarriers are initialised for every thread
-  KWB_STEP_KERNEL_PROLOGUE();
-  const long long t = *S.t0 + step_s;
-  if (mode == KWB_MODE_STEP && t >= S.Nt) return;
-  // once a wait has given up, the simulation is failed: later tiles exit at once instead of each
-  // waiting out its budget (uniform over the CTA: one load before any thread diverges)
-  if (tma && *reinterpret_cast<volatile const int *>(S.err) != 0) return;
+  // The first pass of a step needs the pressure its predecessor wrote (and the step counter that
+  // may just have moved).  The passes after it read nothing of their predecessor but, in XEOS,
+  // its density: they wait there, or after their first transforms, so that in a small grid (512^2:
+  // 128 CTAs a pass) the passes of a step run side by side, and in a large one a pass's first
+  // wave fills its predecessor's tail.
+  const bool wait_first = mode != KWB_MODE_STEP || axis == 1 || S.ndim == 1;
   const int tid = threadIdx.x;
   const int tt = CONTIG ? tid % G : tid / L;
   const int l = CONTIG ? tid / G : tid % L;
@@ -961,12 +982,13 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   // any copy still in flight before the CTA exits.
   bool issued[4] = {false, false, false, false};
   auto tile_wait = [&](int s0, int s1) -> bool {
-    if (!tma) {  // 16-byte cp.async staging: the p tile alone first, then everything
-      if (s0 == 0 && s1 < 0) cp_async_wait<1>();
+    if (!tma) {  // 16-byte cp.async staging: the p tile (and what went before it) first, then everything
+      if (s0 == 0 && s1 < 0 && !wait_first) cp_async_wait<1>();
       else cp_async_wait<0>();
       __syncthreads();
       return true;
     }
+    if (s0 == 0) cp_async_wait<0>();  // the table image
     bool ok = true;
     if (s0 >= 0) ok = mbar_wait_bounded(&tile_bar[s0], 0) && ok;
     if (s1 >= 0) ok = mbar_wait_bounded(&tile_bar[s1], 0) && ok;
@@ -983,18 +1005,70 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     return *reinterpret_cast<const float2 *>(st + i * 2 * L + 2 * l);
   };
   const float *__restrict__ rho0 = S.rho0;
+  // Point sources on this tile's lines (first_order_steps.jl:586-715): the few entries of a tile
+  // are fetched by one thread each while the tile's operands are in flight and wait in shared
+  // memory (entry by entry at the point of use, a chain of three loads each, they held the tiles of
+  // a 9 x 9 disc source up by 3-4 us a pass).  More than SRC_CAP entries on a tile are read in
+  // place.
+  constexpr int SRC_CAP = THREADS < 32 ? THREADS : 32;
+  __shared__ int src_ptr[2][2 * LT + 1];
+  __shared__ int2 src_ent[2][SRC_CAP];  // line << 16 | position, value
+  const bool has_u = mode == KWB_MODE_STEP && S.u_sig[axis] && S.u_line_ptr[axis];
+  const bool has_p = mode == KWB_MODE_STEP && S.n_p > 0 && S.p_line_ptr[axis];
+  int my_j[2] = {-1, -1};
+  auto src_find = [&](int k, const int *lp, const SrcEntry *en) {
+    const int q0 = __ldg(lp + first_line), n = __ldg(lp + first_line + cnt) - q0;
+    for (int c = tid; c <= cnt; c += THREADS) src_ptr[k][c] = __ldg(lp + first_line + c) - q0;
+    if (tid < n && n <= SRC_CAP) {
+      const SrcEntry e = en[q0 + tid];
+      src_ent[k][tid].x = (e.line - first_line) << 16 | e.pos;
+      my_j[k] = e.j;
+    }
+  };
+  if (has_u) src_find(0, S.u_line_ptr[axis], S.u_entry[axis]);
+  if (has_p) src_find(1, S.p_line_ptr[axis], S.p_entry[axis]);
+  if (wait_first) {
+    if (rho0) {
+      stage(st_r, rho0, 1);
+      issued[1] = true;
+    }
+    pdl_wait();
+  }
+  // once a wait has given up, the simulation is failed: later tiles exit at once instead of each
+  // waiting out its budget (uniform over the CTA: one load before any thread diverges)
+  if (tma && *reinterpret_cast<volatile const int *>(S.err) != 0) {
+    for (int b = 0; b < 4; ++b)
+      if (issued[b]) mbar_wait_bounded(&tile_bar[b], 0);
+    cp_async_wait<0>();
+    if (!wait_first) pdl_wait();
+    return;
+  }
   stage(st_p, S.p, 0);
   issued[0] = true;
-  if (rho0) {
-    stage(st_r, rho0, 1);
-    issued[1] = true;
-  } else if (!tma) {
-    cp_async_commit();
+  if (!wait_first) {
+    if (rho0) {
+      stage(st_r, rho0, 1);
+      issued[1] = true;
+    } else if (!tma) {
+      cp_async_commit();
+    }
+  }
+  const long long t = *S.t0 + step_s;
+  if (my_j[0] >= 0) {
+    const int tcol = (int)(min(t + 1, (long long)S.u_cols[axis]) - 1);
+    src_ent[0][tid].y = __float_as_int(S.u_sig[axis][(long long)tcol * S.n_u + my_j[0]]);
+  }
+  if (my_j[1] >= 0) {
+    const int tcol = (int)(min(t + 1, (long long)S.p_cols) - 1);
+    src_ent[1][tid].y = __float_as_int(S.p_sig[(long long)tcol * S.n_p + my_j[1]]);
   }
   float2 *xs = sm + l * LP;
   float *__restrict__ ud = S.u[axis];
   // the p tile has landed (rho0 may still be in flight), for every thread; tables too
-  if (!tile_wait(0, -1)) return;
+  if (!tile_wait(0, -1)) {
+    if (!wait_first) pdl_wait();
+    return;
+  }
   float2 v[E];
 #pragma unroll
   for (int r = 0; r < E; ++r) v[r] = staged(st_p, tt + G * r);
@@ -1012,10 +1086,22 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   for (int q = 0; q < E; ++q) v[q] = cmul(v[q], gp2[q * RP + tt]);
   F::inv(v, xs, tw2, tt);
   // the rho0 and velocity tiles have landed
-  if (!tile_wait(rho0 ? 1 : -1, mode == KWB_MODE_STEP ? 2 : -1)) return;
+  if (!tile_wait(rho0 ? 1 : -1, mode == KWB_MODE_STEP ? 2 : -1)) {
+    if (!wait_first) pdl_wait();
+    return;
+  }
+  if (!XEOS && !wait_first) pdl_wait();
+  if (mode == KWB_MODE_STEP && t >= S.Nt) {
+    if (XEOS && !wait_first) pdl_wait();
+    return;
+  }
 
   // velocity update u = pml_sg (pml_sg u - dt/rho_sg dp)
-  const float *__restrict__ esg = S.pml_sg_def[axis];
+  float pe[PML_S ? 1 : E];  // a batch of deficits, where they are not in shared memory
+  if constexpr (!PML_S) {
+#pragma unroll
+    for (int r = 0; r < E; ++r) pe[r] = __ldg(pml_s + tt + G * r);
+  }
 #pragma unroll
   for (int r = 0; r < E; ++r) {
     const int i = tt + G * r;
@@ -1031,7 +1117,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     if (mode == KWB_MODE_INIT) {
       nv = make_float2(-0.5f * coef.x * v[r].x, -0.5f * coef.y * v[r].y);
     } else {
-      const float2 nes = pair(-__ldg(esg + i));
+      const float2 nes = pair(-(PML_S ? pml_s[i] : pe[PML_S ? 0 : r]));
       const float2 u0 = staged(st_p, i);
       const float2 tu = pfma(make_float2(-coef.x, -coef.y), v[r], pfma(nes, u0, u0));
       nv = pfma(nes, tu, tu);
@@ -1072,26 +1158,36 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     }
   }
 
-  // velocity sources on this tile's lines (first_order_steps.jl:586-617, 646-690)
-  // (entries are sorted by line: a thread scans only its own two lines)
-  if (S.u_sig[axis] && S.u_line_ptr[axis] && va) {
-    const int tcol = (int)(min(t + 1, (long long)S.u_cols[axis]) - 1);
-    const int la = first_line + 2 * l;
-    const int q0 = S.u_line_ptr[axis][la], q1 = S.u_line_ptr[axis][la + (vb ? 2 : 1)];
-    for (int q = q0; q < q1; ++q) {
-      const SrcEntry se = S.u_entry[axis][q];
-      const int c = se.line - la;
-      if ((se.pos % G) != tt) continue;
-      const int ro = se.pos / G;
-      const float val = S.u_sig[axis][(long long)tcol * S.n_u + se.j];
+  // apply the sources of kind K (0 velocity, 1 pressure) on this thread's two lines to v
+  auto src_apply = [&](int K, const int *lp, const SrcEntry *en, const float *sig, int n_sig, int cols, int smode) {
+    auto put = [&](int line, int pos, float val) {
+      if ((pos % G) != tt) return;
+      const int ro = pos / G;
 #pragma unroll
       for (int r = 0; r < E; ++r)
         if (r == ro) {
-          if (c & 1) v[r].y = (S.u_mode == 0) ? val : v[r].y + val;
-          else v[r].x = (S.u_mode == 0) ? val : v[r].x + val;
+          if (line & 1) v[r].y = (smode == 0) ? val : v[r].y + val;
+          else v[r].x = (smode == 0) ? val : v[r].x + val;
         }
+    };
+    const int n = src_ptr[K][cnt], q0 = src_ptr[K][2 * l], q1 = src_ptr[K][2 * l + (vb ? 2 : 1)];
+    if (n <= SRC_CAP) {
+      for (int q = q0; q < q1; ++q) {
+        const int2 e = src_ent[K][q];
+        put(e.x >> 16, e.x & 0xffff, __int_as_float(e.y));
+      }
+    } else {
+      const int tcol = (int)(min(t + 1, (long long)cols) - 1);
+      const SrcEntry *e0 = en + __ldg(lp + first_line);
+      for (int q = q0; q < q1; ++q) {
+        const SrcEntry se = e0[q];
+        if ((se.pos % G) == tt) put(se.line - first_line, se.pos, sig[(long long)tcol * n_sig + se.j]);
+      }
     }
-  }
+  };
+  // velocity sources on this tile's lines (first_order_steps.jl:586-617, 646-690)
+  if (has_u && va)
+    src_apply(0, S.u_line_ptr[axis], S.u_entry[axis], S.u_sig[axis], S.n_u, S.u_cols[axis], S.u_mode);
   float *__restrict__ rd = S.rho[axis];
 #pragma unroll
   for (int r = 0; r < E; ++r) store_pair(ud, tt + G * r, v[r]);
@@ -1102,13 +1198,19 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   for (int q = 0; q < E; ++q) v[q] = cmul(v[q], gn2[q * RP + tt]);
   F::inv(v, xs, tw2, tt);
 
-  if (!tile_wait(3, -1)) return;  // the rho_d tile has landed
+  if (!tile_wait(3, -1)) {  // the rho_d tile has landed
+    if (XEOS && !wait_first) pdl_wait();
+    return;
+  }
   // density update rho_d = pml (pml rho_d - dt rho0 du)
-  const float *__restrict__ ed = S.pml_def[axis];
+  if constexpr (!PML_S) {
+#pragma unroll
+    for (int r = 0; r < E; ++r) pe[r] = __ldg(pml_s + N + tt + G * r);
+  }
 #pragma unroll
   for (int r = 0; r < E; ++r) {
     const int i = tt + G * r;
-    const float2 nei = pair(-__ldg(ed + i));
+    const float2 nei = pair(-(PML_S ? pml_s[N + i] : pe[PML_S ? 0 : r]));
     const float2 ncoef = rho0 ? pmul(pair(-S.dt), staged(st_r, i)) : pair(-S.dt_rho0_s);
     const float2 r0d = staged(st_p, i);
     float2 du = v[r];
@@ -1121,41 +1223,29 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     v[r] = pfma(nei, tr, tr);
   }
   // pressure (mass) sources (first_order_steps.jl:619-640, 692-715)
-  if (S.n_p > 0 && S.p_line_ptr[axis] && va) {
-    const int tcol = (int)(min(t + 1, (long long)S.p_cols) - 1);
-    const int la = first_line + 2 * l;
-    const int q0 = S.p_line_ptr[axis][la], q1 = S.p_line_ptr[axis][la + (vb ? 2 : 1)];
-    for (int q = q0; q < q1; ++q) {
-      const SrcEntry se = S.p_entry[axis][q];
-      const int c = se.line - la;
-      if ((se.pos % G) != tt) continue;
-      const int ro = se.pos / G;
-      const float val = S.p_sig[(long long)tcol * S.n_p + se.j];
-#pragma unroll
-      for (int r = 0; r < E; ++r)
-        if (r == ro) {
-          if (c & 1) v[r].y = (S.p_mode == 0) ? val : v[r].y + val;
-          else v[r].x = (S.p_mode == 0) ? val : v[r].x + val;
-        }
-    }
-  }
+  if (has_p && va) src_apply(1, S.p_line_ptr[axis], S.p_entry[axis], S.p_sig, S.n_p, S.p_cols, S.p_mode);
 #pragma unroll
   for (int r = 0; r < E; ++r) store_pair(rd, tt + G * r, v[r]);
   if constexpr (XEOS) {
     // equation of state, x R2C (k_eos_fwd_fast): sum of the split densities, nonlinearity, c^2
 #pragma unroll
     for (int r = 0; r < E; ++r) v[r] = make_float2(va ? v[r].x : 0.f, vb ? v[r].y : 0.f);
+    if (!wait_first) pdl_wait();  // the other passes' densities
+    auto load_rho = [&](const float *f, int i) -> float2 {
+      const float *fb = f + base;
+      return make_float2(va ? __ldcg(fb + off(2 * l, i)) : 0.f, vb ? __ldcg(fb + off(2 * l + 1, i)) : 0.f);
+    };
     if (S.D > 1) {
 #pragma unroll
       for (int r = 0; r < E; ++r) {
-        const float2 b = load_pair(S.rho[1], tt + G * r);
+        const float2 b = load_rho(S.rho[1], tt + G * r);
         v[r] = padd(v[r], b);
       }
     }
     if (S.D > 2) {
 #pragma unroll
       for (int r = 0; r < E; ++r) {
-        const float2 b = load_pair(S.rho[2], tt + G * r);
+        const float2 b = load_rho(S.rho[2], tt + G * r);
         v[r] = padd(v[r], b);
       }
     }
@@ -1221,10 +1311,11 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   extern __shared__ __align__(128) float4 smem_raw[];
   float2 *sm = reinterpret_cast<float2 *>(smem_raw);
   float2 *tw2 = sm + L * LP;
-  // the twiddles are written once at set-up: built before waiting on the previous kernel
-  F::build_tw(tw2, S.tw[0]);
-  KWB_STEP_KERNEL_PROLOGUE();
+  // the twiddles are written once at set-up: copied before waiting on the previous kernel
+  stage_image(tw2, S.img[0], image_tw_bytes<F>());
+  pdl_wait();
   const long long t = *S.t0 + step_s;
+  cp_async_wait<0>();
   if (t >= S.Nt) return;
   const int tid = threadIdx.x, tt = tid % G, l = tid / G;
   const int Ny = S.N[1];
@@ -1311,11 +1402,8 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   extern __shared__ __align__(128) float4 smem_raw[];
   float2 *sm = reinterpret_cast<float2 *>(smem_raw);
   float2 *tw2 = sm + L * LP;
-  // the twiddles are written once at set-up: built before waiting on the previous kernel
-  F::build_tw(tw2, S.tw[0]);
-  KWB_STEP_KERNEL_PROLOGUE();
-  const long long t = *S.t0 + step_s;
-  if (t >= S.Nt) return;
+  // the twiddles are written once at set-up: copied before waiting on the previous kernel
+  stage_image(tw2, S.img[0], image_tw_bytes<F>());
   const int tid = threadIdx.x, tt = tid % G, l = tid / G;
   const int Ny = S.N[1];
   const int rows = 2 * L, tpp = (Ny + rows - 1) / rows;
@@ -1325,61 +1413,90 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   const bool va = 2 * l < cnt, vb = 2 * l + 1 < cnt;
   float2 *xs = sm + l * LP;
   const int n1 = S.n1;
-  if (PLANE) {
-    // one (kx, line pair) per thread, pairs fastest: the pair's rows are adjacent in y, so A and
-    // B arrive as one 16-byte load and each kx reads 2L consecutive y
-    const int lp = tid % L;
-    float2 *xl = sm + lp * LP;
-    const float2 *srcp = S.spec + ((long long)z * n1 + tid / L) * Ny + y0 + 2 * lp;
-    const long long kstep = (long long)G * Ny;  // THREADS / L = G values of kx per sweep
-    for (int k = tid / L; k < n1; k += G, srcp += kstep) {
-      float2 A = make_float2(0.f, 0.f), B = make_float2(0.f, 0.f);
-      if (2 * lp + 1 < cnt) {
-        const float4 ab = *reinterpret_cast<const float4 *>(srcp);
-        A = make_float2(ab.x, ab.y);
-        B = make_float2(ab.z, ab.w);
-      } else if (2 * lp < cnt) {
-        A = *srcp;
-      }
-      if (k == 0 || 2 * k == N) {
-        xl[F::nat(k)] = make_float2(A.x, B.x);  // c2r ignores Im of the DC and Nyquist bins
-      } else {
-        xl[F::nat(k)] = make_float2(A.x - B.y, A.y + B.x);
-        xl[F::nat(N - k)] = make_float2(A.x + B.y, B.x - A.y);
-      }
-    }
-  } else {
-    const long long rowa = (long long)z * Ny + y0 + 2 * l;
-    for (int k = tt; k < n1; k += G) {
-      const float2 A = va ? S.spec[rowa * n1 + k] : make_float2(0.f, 0.f);
-      const float2 B = vb ? S.spec[(rowa + 1) * n1 + k] : make_float2(0.f, 0.f);
-      if (k == 0 || 2 * k == N) {
-        xs[F::nat(k)] = make_float2(A.x, B.x);  // c2r ignores Im of the DC and Nyquist bins
-      } else {
-        xs[F::nat(k)] = make_float2(A.x - B.y, A.y + B.x);
-        xs[F::nat(N - k)] = make_float2(A.x + B.y, B.x - A.y);
-      }
-    }
-  }
-  __syncthreads();
-  float2 v[E];
-#pragma unroll
-  for (int idx = 0; idx < E; ++idx) v[idx] = xs[F::nat_of(tt, idx)];
-  // dense pressure sensor (record_sensor_data!, first_order_steps.jl:732-752): prefetch the
-  // running max (or, without one, the running min) before the transform, update all fields as p
-  // is written.  One prefetched field keeps the kernel within its register budget.
+  // what this pass reads of the simulation's set-up or of its own last step (sensor records, the
+  // running max or min) is read before waiting on the previous kernel
   const GroupDev *gd = S.dense_p;
   const unsigned gm = gd ? gd->mask : 0u;
   constexpr bool PFS = E <= 16;  // prefetch only while it fits in registers
   float2 pm[PFS ? E : 1];
   const bool pf_max = PFS && (gm & (1u << 1)), pf_min = PFS && !pf_max && (gm & (1u << 2));
   const long long ra = base + (long long)(2 * l) * N, rb = ra + N;
+  const GroupDev *gs = S.sparse_p;
+  int qa = 0, qb = 0, qc = 0;
+  if (gs && va) {
+    const int *lp = gs->line_ptr + (z * Ny + y0 + 2 * l);
+    qa = __ldg(lp);
+    qb = __ldg(lp + 1);
+    qc = vb ? __ldg(lp + 2) : qb;
+  }
+  pdl_wait();
+  const long long t = *S.t0 + step_s;
+  // The half spectrum's rows, all of a thread's loads in flight at once (k = tt + G j, and the
+  // Nyquist bin): issued one by one between the stores they feed, they took 2 us of a 512^2 pass.
+  constexpr int KJ = E / 2;
+  static_assert(E % 2 == 0, "the half spectrum is KJ bins per thread and the Nyquist bin");
+  auto unpack = [&](float2 *x, int k, float2 A, float2 B) {
+    if (k == 0 || 2 * k == N) {
+      x[F::nat(k)] = make_float2(A.x, B.x);  // c2r ignores Im of the DC and Nyquist bins
+    } else {
+      x[F::nat(k)] = make_float2(A.x - B.y, A.y + B.x);
+      x[F::nat(N - k)] = make_float2(A.x + B.y, B.x - A.y);
+    }
+  };
+  float4 ab[KJ];
+  float4 nyq = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (PLANE) {
+    // one (kx, line pair) per thread, pairs fastest: the pair's rows are adjacent in y, so A and
+    // B arrive as one 16-byte load and each kx reads 2L consecutive y
+    const int lp = tid % L, kk = tid / L;
+    float2 *xl = sm + lp * LP;
+    const float2 *srcp = S.spec + ((long long)z * n1 + kk) * Ny + y0 + 2 * lp;
+    const long long kstep = (long long)G * Ny;  // THREADS / L = G values of kx per sweep
+    auto ld = [&](const float2 *q) -> float4 {
+      if (2 * lp + 1 < cnt) return __ldcg(reinterpret_cast<const float4 *>(q));
+      if (2 * lp < cnt) {
+        const float2 A = __ldcg(q);
+        return make_float4(A.x, A.y, 0.f, 0.f);
+      }
+      return make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) ab[j] = ld(srcp + j * kstep);
+    if (kk == 0) nyq = ld(srcp + KJ * kstep);
+#pragma unroll
+    for (int j = 0; j < KJ; ++j)
+      unpack(xl, kk + G * j, make_float2(ab[j].x, ab[j].y), make_float2(ab[j].z, ab[j].w));
+    if (kk == 0) unpack(xl, N / 2, make_float2(nyq.x, nyq.y), make_float2(nyq.z, nyq.w));
+  } else {
+    const float2 *sa = S.spec + ((long long)z * Ny + y0 + 2 * l) * n1, *sb = sa + n1;
+    auto ld = [&](int k) -> float4 {
+      const float2 A = va ? __ldcg(sa + k) : make_float2(0.f, 0.f);
+      const float2 B = vb ? __ldcg(sb + k) : make_float2(0.f, 0.f);
+      return make_float4(A.x, A.y, B.x, B.y);
+    };
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) ab[j] = ld(tt + G * j);
+    if (tt == 0) nyq = ld(N / 2);
+#pragma unroll
+    for (int j = 0; j < KJ; ++j)
+      unpack(xs, tt + G * j, make_float2(ab[j].x, ab[j].y), make_float2(ab[j].z, ab[j].w));
+    if (tt == 0) unpack(xs, N / 2, make_float2(nyq.x, nyq.y), make_float2(nyq.z, nyq.w));
+  }
+  cp_async_wait<0>();
+  __syncthreads();  // the spectrum and the twiddles
+  if (t >= S.Nt) return;
+  float2 v[E];
+#pragma unroll
+  for (int idx = 0; idx < E; ++idx) v[idx] = xs[F::nat_of(tt, idx)];
+  // dense pressure sensor (record_sensor_data!, first_order_steps.jl:732-752): the running max
+  // (or, without one, the running min) is loaded under the transform, all fields are updated as p
+  // is written.  One prefetched field keeps the kernel within its register budget.
   if (pf_max || pf_min) {
     const float *pa = pf_max ? gd->pmax : gd->pmin;
 #pragma unroll
     for (int r = 0; r < E; ++r) {
       const int i = tt + G * r;
-      pm[PFS ? r : 0] = make_float2(va ? pa[ra + i] : 0.f, vb ? pa[rb + i] : 0.f);
+      pm[PFS ? r : 0] = make_float2(va ? __ldcg(pa + ra + i) : 0.f, vb ? __ldcg(pa + rb + i) : 0.f);
     }
   }
   F::sync();
@@ -1414,13 +1531,26 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
       }
     }
     if (gm & (1u << 3)) {
+      // (a batch of sums is loaded before the first is stored: alternating, each load waited for
+      // the store before it, 3.3 us of a 512^2 pass)
       double *a = gd->prms + ra;
       const double w = (double)gd->cnt_prms;
+      constexpr int RB = E % 4 == 0 ? 4 : 2;
 #pragma unroll
-      for (int r = 0; r < E; ++r) {
-        const int i = tt + G * r;
-        if (va) a[i] += w * ((double)v[r].x * (double)v[r].x);
-        if (vb) a[N + i] += w * ((double)v[r].y * (double)v[r].y);
+      for (int r0 = 0; r0 < E; r0 += RB) {
+        double qa2[RB], qb2[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+          const int i = tt + G * (r0 + r);
+          qa2[r] = va ? __ldcg(a + i) : 0.0;
+          qb2[r] = vb ? __ldcg(a + N + i) : 0.0;
+        }
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+          const int i = tt + G * (r0 + r);
+          if (va) a[i] = qa2[r] + w * ((double)v[r0 + r].x * (double)v[r0 + r].x);
+          if (vb) a[N + i] = qb2[r] + w * ((double)v[r0 + r].y * (double)v[r0 + r].y);
+        }
       }
     }
     if ((gm & (1u << 4)) && t == S.Nt - 1) put(gd->pfinal + ra);
@@ -1428,12 +1558,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   // sparse pressure sensor (record_sensor_data!, first_order_steps.jl:732-752): this thread's
   // p values go to its line's exchange buffer (x order, the two rows as one pair), then the
   // points on the line pair are recorded from there through the group's per-x-line index
-  const GroupDev *gs = S.sparse_p;
   if (gs) {
-    const int line0 = z * Ny + y0 + 2 * l;
-    const int qa = va ? gs->line_ptr[line0] : 0;
-    const int qb = va ? gs->line_ptr[line0 + 1] : 0;
-    const int qc = vb ? gs->line_ptr[line0 + 2] : qb;
     // most lines hold no point: skip the exchange unless some line of the group (the warp for
     // one-warp lines, else the block) does
     bool any = qc > qa;
@@ -1471,11 +1596,8 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   extern __shared__ __align__(128) float4 smem_raw[];
   float2 *sm = reinterpret_cast<float2 *>(smem_raw);
   float2 *tw2 = sm + L * LP;
-  // the twiddles are written once at set-up: built before waiting on the previous kernel
-  F::build_tw(tw2, S.tw[axis]);
-  KWB_STEP_KERNEL_PROLOGUE();
-  const long long t = *S.t0 + step_s;
-  if (t >= S.Nt) return;
+  // the twiddles are written once at set-up: copied before waiting on the previous kernel
+  stage_image(tw2, S.img[axis], image_tw_bytes<F>());
   const int tid = threadIdx.x, l = tid % L, tt = tid / L;
   const int n1 = S.n1, Ny = S.N[1];
   const int tpp = (n1 + L - 1) / L;
@@ -1493,15 +1615,31 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   float2 *xs = sm + l * LP;
   float2 *__restrict__ spec = S.spec;
   float2 v[E];
+  // so is the multiplier
+  float m[E];
+  if (op == KWB_SPEC_FWD_MUL_INV) {
+#pragma unroll
+    for (int idx = 0; idx < E; ++idx) {
+      const int k = F::k_of(tt, idx);
+      const long long mi = (axis == 1) ? ((long long)o * Ny + k) * n1 + k0 + l
+                                       : ((long long)k * Ny + o) * n1 + k0 + l;
+      m[idx] = valid ? __ldg(S.M + mi) : 0.f;
+    }
+  }
+  pdl_wait();
+  const long long t = *S.t0 + step_s;
   if (op == KWB_SPEC_INV) {
 #pragma unroll
     for (int idx = 0; idx < E; ++idx)
-      v[idx] = valid ? spec[base + (long long)F::k_of(tt, idx) * stride] : make_float2(0.f, 0.f);
+      v[idx] = valid ? __ldcg(spec + base + (long long)F::k_of(tt, idx) * stride) : make_float2(0.f, 0.f);
   } else {
 #pragma unroll
-    for (int r = 0; r < E; ++r) v[r] = valid ? spec[base + (long long)(tt + G * r) * stride] : make_float2(0.f, 0.f);
+    for (int r = 0; r < E; ++r)
+      v[r] = valid ? __ldcg(spec + base + (long long)(tt + G * r) * stride) : make_float2(0.f, 0.f);
   }
+  cp_async_wait<0>();
   __syncthreads();
+  if (t >= S.Nt) return;
   if (op == KWB_SPEC_INV) {
     F::inv(v, xs, tw2, tt);
   } else {
@@ -1514,13 +1652,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
       return;
     }
 #pragma unroll
-    for (int idx = 0; idx < E; ++idx) {
-      const int k = F::k_of(tt, idx);
-      const long long mi = (axis == 1) ? ((long long)o * Ny + k) * n1 + k0 + l
-                                       : ((long long)k * Ny + o) * n1 + k0 + l;
-      const float m = valid ? __ldg(S.M + mi) : 0.f;
-      v[idx] = cscale(v[idx], m);
-    }
+    for (int idx = 0; idx < E; ++idx) v[idx] = cscale(v[idx], m[idx]);
     F::inv(v, xs, tw2, tt);
   }
   if (valid) {
@@ -1586,10 +1718,10 @@ __global__ void __launch_bounds__(THREADS, MINB)
   float2 *xsb = data + RZ * NY;
   float2 *twy = xsb + XS;
   float2 *twz = twy + FY::TW;
-  // the twiddles are written once at set-up: built before waiting on the previous kernel
-  FY::build_tw(twy, S.tw[1]);
-  FZ::build_tw(twz, S.tw[2]);
-  KWB_STEP_KERNEL_PROLOGUE();
+  // the twiddles are written once at set-up: copied before waiting on the previous kernel
+  stage_image(twy, S.img[1], FY::TW * sizeof(float2));
+  stage_image(twz, S.img[2], FZ::TW * sizeof(float2));
+  pdl_wait();
   const long long t = *S.t0 + step_s;
   if (t >= S.Nt) return;  // uniform over the cluster
   const unsigned rank = cluster_rank();
@@ -1698,16 +1830,16 @@ __global__ void __launch_bounds__(THREADS, MINB)
     k_plane_cols(const __grid_constant__ SimDev S, long long step_s) {
   constexpr int NY = F::N, NZ = F::N, RZ = NZ / CL, CY = NY / CL, W = THREADS / 32;
   constexpr int RP = RZ + 1;  // pitch of a slot column (odd: conflict-free row stores)
-  static_assert(F::G == 32 && F::WARP_SYNC, "one warp per line");
+  static_assert(F::G == 32 && F::WARP_SYNC && F::TW % 2 == 0, "one warp per line");
   static_assert(RZ % W == 0 && CY % W == 0 && NZ % RZ == 0, "plane tiling");
   extern __shared__ __align__(128) float4 smem_raw[];
   float2 *cols = reinterpret_cast<float2 *>(smem_raw);  // [NY][RP]
   float2 *xsb = cols + NY * RP;                          // one exchange buffer per warp
   float2 *twy = xsb + W * F::LP;
   float2 *twz = twy + F::TW;
-  F::build_tw(twy, S.tw[1]);
-  F::build_tw(twz, S.tw[2]);
-  KWB_STEP_KERNEL_PROLOGUE();
+  stage_image(twy, S.img[1], F::TW * sizeof(float2));
+  stage_image(twz, S.img[2], F::TW * sizeof(float2));
+  pdl_wait();
   const long long t = *S.t0 + step_s;
   if (t >= S.Nt) return;  // uniform over the cluster
   const unsigned rank = cluster_rank();
@@ -1718,6 +1850,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   if (S.eos_prefetch && threadIdx.x == 0) bulk_prefetch_l2(Mk + (long long)rank * CY * NZ, (unsigned)(CY * NZ * 4));
   const long long rstride = (long long)S.n1 * NY;  // between consecutive z rows of the plane
   float2 *plane = S.spec + (long long)rank * RZ * rstride + (long long)kx * NY;
+  cp_async_wait<0>();
   __syncthreads();  // twiddles
 
   // 1. forward along y, rows to slot-major columns
@@ -1940,6 +2073,17 @@ static inline cudaError_t prime_line_variant() {
     if (e == cudaSuccess) e = raise_smem((const void *)k_line_fast<F, C, LT, P::MINB, false, true>, pline_smem<F>(LT));
   }
   return e;
+}
+
+// Table image of a line length (k_build_image).
+template <int N>
+static inline cudaError_t image_n(float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                                  const float *pml_sg, const float *pml, cudaStream_t st) {
+  using F = typename LinePolicy<N>::template F<false>;
+  if (bytes) *bytes = image_bytes<F>();
+  if (!img) return cudaSuccess;
+  k_build_image<F><<<1, 256, 0, st>>>(img, tw, gpos, gneg, pml_sg, pml);
+  return cudaGetLastError();
 }
 
 template <int N>
@@ -2206,9 +2350,11 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   float2 *tw2 = sm + L * LP;
   float2 *gp2 = tw2 + F::TW;
   float2 *gn2 = gp2 + E * RP;
-  build_line_tables<F>(tw2, gp2, gn2, S.tw[axis], S.gpos[axis], S.gneg[axis]);
-  KWB_STEP_KERNEL_PROLOGUE();
-  if (*S.t0 + step_s >= S.Nt) return;
+  stage_image(tw2, S.img[axis], image_line_bytes<F>());
+  // the first pass of a group (x) transforms what its predecessor wrote; the others only add to it,
+  // and wait for it after their first transform
+  const bool wait_first = axis == 0;
+  if (wait_first) pdl_wait();
   const int tid = threadIdx.x;
   const int tt = CONTIG ? tid % G : tid / L;
   const int l = CONTIG ? tid / G : tid % L;
@@ -2272,8 +2418,8 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   // the destination as this kernel may already have written it: ordinary (coherent) loads
   auto load_cur = [&](const float *f, int i) -> float2 {
     const float *fb = f + base;
-    if (!CONTIG) return vb ? *reinterpret_cast<const float2 *>(fb + off(2 * l, i)) : make_float2(0.f, 0.f);
-    return make_float2(va ? fb[off(2 * l, i)] : 0.f, vb ? fb[off(2 * l + 1, i)] : 0.f);
+    if (!CONTIG) return vb ? __ldcg(reinterpret_cast<const float2 *>(fb + off(2 * l, i))) : make_float2(0.f, 0.f);
+    return make_float2(va ? __ldcg(fb + off(2 * l, i)) : 0.f, vb ? __ldcg(fb + off(2 * l + 1, i)) : 0.f);
   };
   auto store_pair = [&](float *f, int i, float2 v) {
     float *fb = f + base;
@@ -2297,6 +2443,8 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     float2 v[E];
 #pragma unroll
     for (int r = 0; r < E; ++r) v[r] = staged(slot, tt + G * r);
+    if (f == 0 && !wait_first) pdl_wait();
+    if (f == 0 && *S.t0 + step_s >= S.Nt) break;
     if (f + 2 < g.nf) {
       __syncthreads();  // every thread holds field f
       stage(slot, g.src[f + 2]);

@@ -23,6 +23,10 @@ cudaError_t fast_mixed_prime(int N) {
   cudaError_t e = prime_eos_mixed(N);
   return e != cudaSuccess ? e : prime_line_mixed(N);
 }
+cudaError_t fast_mixed_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                     const float *pml_sg, const float *pml, cudaStream_t st) {
+  KWB_MIXED_SWITCH(N, image_n, (img, bytes, tw, gpos, gneg, pml_sg, pml, st))
+}
 cudaError_t fast_mixed_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                                  cudaStream_t st) {
   KWB_MIXED_SWITCH(h.N[axis], launch_line_n, (d_sim, h, axis, mode, s, st))

@@ -22,6 +22,10 @@ cudaError_t fast_mixed2_prime(int N) {
   cudaError_t e = prime_eos_mixed2(N);
   return e != cudaSuccess ? e : prime_line_mixed2(N);
 }
+cudaError_t fast_mixed2_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                     const float *pml_sg, const float *pml, cudaStream_t st) {
+  KWB_MIXED2_SWITCH(N, image_n, (img, bytes, tw, gpos, gneg, pml_sg, pml, st))
+}
 cudaError_t fast_mixed2_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                                  cudaStream_t st) {
   KWB_MIXED2_SWITCH(h.N[axis], launch_line_n, (d_sim, h, axis, mode, s, st))

@@ -21,6 +21,10 @@ cudaError_t fast_mixed4_prime(int N) {
   cudaError_t e = prime_eos_mixed4(N);
   return e != cudaSuccess ? e : prime_line_mixed4(N);
 }
+cudaError_t fast_mixed4_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                     const float *pml_sg, const float *pml, cudaStream_t st) {
+  KWB_MIXED4_SWITCH(N, image_n, (img, bytes, tw, gpos, gneg, pml_sg, pml, st))
+}
 cudaError_t fast_mixed4_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                                  cudaStream_t st) {
   KWB_MIXED4_SWITCH(h.N[axis], launch_line_n, (d_sim, h, axis, mode, s, st))

@@ -118,6 +118,7 @@ struct SimDev {
   const float2 *gpos[3];
   const float2 *gneg[3];
   const float2 *tw[3];
+  const float2 *img[3];  // table image of each register-FFT axis (fast_image), nullptr otherwise
   FftPlan plan[3];
 
   // tile shapes: complex lines per tile for line passes (per axis), x-direction EOS passes and
@@ -294,6 +295,8 @@ struct ElGrad;
 bool fast_size(int N);
 bool fast_mixed_size(int N);
 cudaError_t fast_mixed_prime(int N);
+cudaError_t fast_mixed_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                     const float *pml_sg, const float *pml, cudaStream_t st);
 cudaError_t fast_mixed_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                                  cudaStream_t st);
 cudaError_t fast_mixed_eos(const SimDev *d_sim, const SimDev &h, bool fwd, long long s, cudaStream_t st);
@@ -303,6 +306,8 @@ cudaError_t fast_mixed_el_grad(const SimDev &h, int axis, const ElGrad &g, long 
 // ... and (kwb_fast_mixed2.cu) 80, 384, 640, 768.
 bool fast_mixed2_size(int N);
 cudaError_t fast_mixed2_prime(int N);
+cudaError_t fast_mixed2_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                     const float *pml_sg, const float *pml, cudaStream_t st);
 cudaError_t fast_mixed2_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                                   cudaStream_t st);
 cudaError_t fast_mixed2_eos(const SimDev *d_sim, const SimDev &h, bool fwd, long long s, cudaStream_t st);
@@ -312,6 +317,8 @@ cudaError_t fast_mixed2_el_grad(const SimDev &h, int axis, const ElGrad &g, long
 // ... (kwb_fast_mixed3.cu) 144, 288, 432.
 bool fast_mixed3_size(int N);
 cudaError_t fast_mixed3_prime(int N);
+cudaError_t fast_mixed3_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                     const float *pml_sg, const float *pml, cudaStream_t st);
 cudaError_t fast_mixed3_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                                   cudaStream_t st);
 cudaError_t fast_mixed3_eos(const SimDev *d_sim, const SimDev &h, bool fwd, long long s, cudaStream_t st);
@@ -321,6 +328,8 @@ cudaError_t fast_mixed3_el_grad(const SimDev &h, int axis, const ElGrad &g, long
 // ... (kwb_fast_mixed4.cu) 576, 864, 400.
 bool fast_mixed4_size(int N);
 cudaError_t fast_mixed4_prime(int N);
+cudaError_t fast_mixed4_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                     const float *pml_sg, const float *pml, cudaStream_t st);
 cudaError_t fast_mixed4_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                                   cudaStream_t st);
 cudaError_t fast_mixed4_eos(const SimDev *d_sim, const SimDev &h, bool fwd, long long s, cudaStream_t st);
@@ -330,6 +339,8 @@ cudaError_t fast_mixed4_el_grad(const SimDev &h, int axis, const ElGrad &g, long
 // ... (kwb_fast_mixed5.cu) 500, 800, 1000.
 bool fast_mixed5_size(int N);
 cudaError_t fast_mixed5_prime(int N);
+cudaError_t fast_mixed5_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                     const float *pml_sg, const float *pml, cudaStream_t st);
 cudaError_t fast_mixed5_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                                   cudaStream_t st);
 cudaError_t fast_mixed5_eos(const SimDev *d_sim, const SimDev &h, bool fwd, long long s, cudaStream_t st);
@@ -337,6 +348,9 @@ cudaError_t fast_mixed5_spec(const SimDev *d_sim, const SimDev &h, int axis, int
                              cudaStream_t st);
 cudaError_t fast_mixed5_el_grad(const SimDev &h, int axis, const ElGrad &g, long long s, cudaStream_t st);
 cudaError_t fast_prime(int N);
+// Table image of a register-FFT axis: its size in bytes, and (img not null) its contents.
+cudaError_t fast_image(int N, float2 *img, size_t *bytes, const float2 *tw, const float2 *gpos, const float2 *gneg,
+                       const float *pml_sg, const float *pml, cudaStream_t st);
 cudaError_t fast_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode, long long s,
                            cudaStream_t st);
 cudaError_t fast_eos(const SimDev *d_sim, const SimDev &h, bool fwd, long long s, cudaStream_t st);
