@@ -600,35 +600,16 @@ cudaError_t elastic_step(kwb_sim *S, long long s, Run &&run) {
   cudaError_t e;
   // stress divergence: the pass along d adds d/dx_d sigma_dj to w_j
   for (int d = 0; d < D; ++d) {
-    ElGrad g{};
-    g.nf = D;
-    for (int j = 0; j < D; ++j) {
-      g.src[j] = h.el_s[kwb_stress_slot(d, j)];
-      g.dst[j] = h.el_w[j];
-    }
-    g.acc = d > 0 ? 7 : 0;
-    g.neg = 0;
+    const ElGrad g = el_stress_grad(h, d);
     if ((e = run(gname[0][d], nv * 4.0 * D * (d > 0 ? 3 : 2), [&] { return el_grad(h, d, g, s, st); })) != cudaSuccess)
       return e;
   }
   if ((e = run("el_velocity", nv * 4.0 * (3 * D + (h.rho0 ? 2 : 0)), [&] { return el_velocity(h, s, st); })) != cudaSuccess)
     return e;
   if (h.n_u > 0 && (e = run("el_inject", 0.0, [&] { return el_inject(h, 0, s, st); })) != cudaSuccess) return e;
-  // velocity gradients: dv_d/dx_d into w_d, dv_j/dx_d into the shear slot {d, j} (first writer
-  // is the pass along the smaller axis, the other adds)
   for (int d = 0; d < D; ++d) {
-    ElGrad g{};
-    g.nf = D;
-    int reads = D;
-    for (int j = 0; j < D; ++j) {
-      g.src[j] = h.u[j];
-      g.dst[j] = h.el_w[kwb_stress_slot(d, j)];
-      if (j < d) {
-        g.acc |= 1 << j;
-        ++reads;
-      }
-    }
-    g.neg = 1;
+    const ElGrad g = el_velocity_grad(h, d);
+    const int reads = D + d;  // d of the destinations are added to
     if ((e = run(gname[1][d], nv * 4.0 * (reads + D), [&] { return el_grad(h, d, g, s, st); })) != cudaSuccess)
       return e;
   }
@@ -875,9 +856,9 @@ static std::string sched_key(int device, const SimDev &h) {
   if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) snprintf(name, sizeof(name), "%s/%d", prop.name, prop.multiProcessorCount);
   char buf[512];
   const char *eo = getenv("KWB_TUNE_ORDER");
-  snprintf(buf, sizeof(buf), "%.200s|v%d.%d|nd%d|N%dx%dx%d|fast%d|plane%d|fuse%d|disp%d|fill%d|axi%d|rho%d|c%d|nl%d|ord%d",
+  snprintf(buf, sizeof(buf), "%.200s|v%d.%d|nd%d|N%dx%dx%d|fast%d|plane%d|fuse%d|disp%d|fill%d|axi%d|el%d|rho%d|c%d|nl%d|ord%d",
            name, KWB_VERSION, KWB_SCHED_GEN, h.ndim, h.N[0], h.N[1], h.N[2], h.fast, h.plane, h.fuse_xeos, h.dispersion,
-           h.grid_fill, h.inv_r ? 1 : 0, h.rho0 ? 1 : 0, h.c0sq ? 1 : 0, (h.nonlinear && h.nlq) ? 2 : h.nonlinear,
+           h.grid_fill, h.inv_r ? 1 : 0, h.elastic, h.rho0 ? 1 : 0, h.c0sq ? 1 : 0, (h.nonlinear && h.nlq) ? 2 : h.nonlinear,
            (eo && strcmp(eo, "1") == 0) ? 1 : 0);
   return buf;
 }
@@ -917,8 +898,10 @@ static int choose_schedule(kwb_sim *S, SimDev &h, cudaStream_t st) {
   CU(cudaMemsetAsync(h.p, 0, nvox * 4, st));
   for (int a = 0; a < h.D; ++a) {
     CU(cudaMemsetAsync(h.u[a], 0, nvox * 4, st));
-    CU(cudaMemsetAsync(h.rho[a], 0, nvox * 4, st));
+    if (h.rho[a]) CU(cudaMemsetAsync(h.rho[a], 0, nvox * 4, st));
   }
+  for (float *f : h.el_s)
+    if (f) CU(cudaMemsetAsync(f, 0, nvox * 4, st));
   if (h.spec) CU(cudaMemsetAsync(h.spec, 0, h.nspec * sizeof(float2), st));
   if (h.spec2) CU(cudaMemsetAsync(h.spec2, 0, h.nspec * sizeof(float2), st));
   if (h.rho_prev) CU(cudaMemsetAsync(h.rho_prev, 0, nvox * 4, st));
@@ -1585,9 +1568,9 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   slog.mark("tr+dense");
   // ---- FFT schedule: measured on first use of this shape (simulations of the batching
   // scheduler share the GPU with others, so they keep the heuristic)
-  if (!h.elastic && !ctx->batched && S->Nt_loop > 0) {
+  if (!ctx->batched && S->Nt_loop > 0) {
     if ((rc = choose_schedule(S.get(), h, st))) return rc;
-    CU(prime_attributes(h));
+    CU(h.elastic ? el_prime(h) : prime_attributes(h));
   }
   if (!h.elastic) {
     // [kz][ky][kx]; with the plane pass [kx][kz][slot], or [kx][slot][k_z in register order]

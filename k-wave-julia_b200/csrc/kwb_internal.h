@@ -382,6 +382,31 @@ struct ElGrad {
   int acc;  // bit f: dst[f] += d/dx_axis src[f]; else dst[f] = d/dx_axis src[f]
   int neg;  // 1: staggered - (velocity gradients), 0: staggered + (stress gradients)
 };
+// The passes of a step along axis d: the stress divergence (d/dx_d sigma_dj added to w_j), and the
+// velocity gradients (dv_d/dx_d into w_d, dv_j/dx_d into the shear slot {d, j}: its first writer is
+// the pass along the smaller axis, the other adds).
+inline ElGrad el_stress_grad(const SimDev &h, int d) {
+  ElGrad g{};
+  g.nf = h.ndim;
+  for (int j = 0; j < h.ndim; ++j) {
+    g.src[j] = h.el_s[kwb_stress_slot(d, j)];
+    g.dst[j] = h.el_w[j];
+  }
+  g.acc = d > 0 ? 7 : 0;
+  g.neg = 0;
+  return g;
+}
+inline ElGrad el_velocity_grad(const SimDev &h, int d) {
+  ElGrad g{};
+  g.nf = h.ndim;
+  for (int j = 0; j < h.ndim; ++j) {
+    g.src[j] = h.u[j];
+    g.dst[j] = h.el_w[kwb_stress_slot(d, j)];
+    if (j < d) g.acc |= 1 << j;
+  }
+  g.neg = 1;
+  return g;
+}
 cudaError_t el_prime(const SimDev &h);
 cudaError_t el_grad(const SimDev &h, int axis, const ElGrad &g, long long s, cudaStream_t st);
 cudaError_t el_velocity(const SimDev &h, long long s, cudaStream_t st);

@@ -114,7 +114,7 @@ struct Tuner {
   template <class F>
   float time(F go) {
     cudaError_t e = cudaMemcpyAsync(d_t, &t, sizeof(SimDev), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = prime_attributes(t);
+    if (e == cudaSuccess) e = t.elastic ? el_prime(t) : prime_attributes(t);
     if (e == cudaSuccess) e = go();
     if (e == cudaSuccess) e = cudaEventRecord(e0, st);
     for (int r = 0; r < 3 && e == cudaSuccess; ++r) e = go();
@@ -203,6 +203,14 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
   // own pass alone: a pass's tile shape also changes how its launch overlaps its neighbours'.
   auto step = [&]() -> cudaError_t {
     cudaError_t e;
+    if (t.elastic) {
+      for (int d2 = 0; d2 < D; ++d2)
+        if ((e = el_grad(t, d2, el_stress_grad(t, d2), 0, st)) != cudaSuccess) return e;
+      if ((e = el_velocity(t, 0, st)) != cudaSuccess) return e;
+      for (int d2 = 0; d2 < D; ++d2)
+        if ((e = el_grad(t, d2, el_velocity_grad(t, d2), 0, st)) != cudaSuccess) return e;
+      return el_stress(t, 0, st);
+    }
     for (int a : {1, 2, 0})
       if (a < D && (e = launch_line_pass(d, t, a, KWB_MODE_STEP, 0, st)) != cudaSuccess) return e;
     if (!t.fuse_xeos && (e = launch_eos_x_fwd(d, t, 0, st)) != cudaSuccess) return e;
@@ -223,6 +231,7 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
     auto go = step;
     if (line_is_fast(t, a)) {
       T.choose("line_tile", 3, [&, a](int i) { t.tile_var[KWB_SLOT_LINE0 + a] = (signed char)i; }, go);
+      if (t.elastic) continue;  // its gradient passes stage by cp.async
       // tiles staged by TMA copies or by 16-byte cp.async (unless KWB_TILE_TMA fixes it)
       if (!getenv("KWB_TILE_TMA"))
         T.choose("line_tma", 2, [&, a](int i) { t.tma_line[a] = (signed char)(i == 0 ? 0 : 1); }, go);
@@ -253,7 +262,7 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
   }
 
   // equation of state, x direction
-  if (D >= 1) {
+  if (!t.elastic) {
     if (eos_is_fast(t)) {
       if (!t.fuse_xeos)
         T.choose("eos_fwd_tile", 3, [&](int i) { t.tile_var[KWB_SLOT_EOS_FWD] = (signed char)i; },
@@ -277,7 +286,7 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
              step);
   }
   // spectrum passes along y and z
-  if (!t.plane) {
+  if (!t.plane && !t.elastic) {
     for (int a = 1; a < D; ++a) {
       auto go = step;
       if (spec_is_fast(t, a)) {
