@@ -7,6 +7,7 @@
 // kwb_kernels.cu; elastic problems step through elastic_step (kernels in kwb_elastic.cu).
 #include <algorithm>
 #include <cmath>
+#include <complex>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -148,125 +149,214 @@ double pairwise_sum(const double *x, long long n, int par = 0) {
 
 namespace kwb {
 
-// Stockham stage radices of a line of N points: 8s first, then 4 or 2, then 3, 5, 7.
+namespace {
+
+// The fewest radices with product n, no radix above `top` (then the smallest largest one, then the
+// smallest sum); cur: the radices so far, best: the best so far.
+void pick_radices(int n, int top, bool prime_only, std::vector<int> &cur, std::vector<int> &best, bool &found) {
+  if (n == 1) {
+    auto sum = [](const std::vector<int> &v) {
+      int t = 0;
+      for (int r : v) t += r;
+      return t;
+    };
+    const bool better = !found || cur.size() < best.size() ||
+                        (cur.size() == best.size() &&
+                         (cur.empty() || cur[0] < best[0] || (cur[0] == best[0] && sum(cur) < sum(best))));
+    if (better) {
+      best = cur;
+      found = true;
+    }
+    return;
+  }
+  if (found && cur.size() >= best.size()) return;
+  static const int radices[] = {16, 15, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  static const int primes[] = {13, 11, 7, 5, 4, 3, 2};
+  for (int k = 0; k < (prime_only ? 7 : 14); ++k) {
+    const int r = prime_only ? primes[k] : radices[k];
+    if (r > top || n % r) continue;
+    cur.push_back(r);  // descending
+    pick_radices(n / r, r, prime_only, cur, best, found);
+    cur.pop_back();
+  }
+}
+
+int largest_prime(int n) {
+  int best = 1;
+  for (int p = 2; p * p <= n; ++p)
+    while (n % p == 0) {
+      best = std::max(best, p);
+      n /= p;
+    }
+  return std::max(best, n);
+}
+
+}  // namespace
+
 bool make_plan_order(int N, FftPlan &pl, int order) {
   pl.n = N;
   pl.nstages = 0;
-  int n = N, a = 0;
-  while (n % 2 == 0) {
-    n /= 2;
-    ++a;
-  }
-  int odd[KWB_MAX_STAGES], nodd = 0;
-  for (int p : {3, 5, 7}) {
-    while (n % p == 0) {
-      if (nodd >= KWB_MAX_STAGES) return false;
-      odd[nodd++] = p;
-      n /= p;
-    }
-  }
-  if (n != 1) return false;
-  auto push = [&](int r) {
-    if (pl.nstages >= KWB_MAX_STAGES) return false;
-    pl.radix[pl.nstages++] = r;
-    return true;
-  };
-  if (order == 2)
-    for (int i = 0; i < nodd; ++i)
-      if (!push(odd[i])) return false;
-  const int big = order == 1 ? 2 : 3;  // log2 of the largest power-of-two radix
-  while (a >= big)
-    if (!push(1 << big)) return false;
-    else a -= big;
-  if (a == 2 && !push(4)) return false;
-  if (a == 1 && !push(2)) return false;
-  if (order != 2)
-    for (int i = 0; i < nodd; ++i)
-      if (!push(odd[i])) return false;
-  // the stages' divisions by the butterflies per line and by the sub-transform length so far
-  int ns = 1;
-  for (int st = 0; st < pl.nstages; ++st) {
-    pl.div_nr[st] = make_fastdiv((unsigned)(N / pl.radix[st]));
-    pl.div_ns[st] = make_fastdiv((unsigned)ns);
-    ns *= pl.radix[st];
+  std::vector<int> cur, r;
+  bool found = false;
+  pick_radices(N, N, order == 1, cur, r, found);
+  if (!found || r.size() > KWB_MAX_STAGES - 1) return false;
+  if (order != 2) std::reverse(r.begin(), r.end());
+  // an odd radix last, where there is one: the last stage's butterflies lie R positions apart, which
+  // then fall in distinct banks
+  if (order != 1)
+    for (size_t k = r.size(); k-- > 0;)
+      if (r[k] % 2) {
+        std::rotate(r.begin() + k, r.begin() + k + 1, r.end());
+        break;
+      }
+  while (r.size() < 2) r.insert(r.begin(), 1);
+  int len = N;  // of the sub-transforms at each stage
+  for (int R : r) {
+    const int st = pl.nstages++;
+    pl.radix[st] = R;
+    pl.stride[st] = len / R;
+    pl.tstride[st] = N / len;
+    pl.nbf[st] = N / R;
+    pl.div_st[st] = make_fastdiv((unsigned)(len / R));
+    pl.div_r[st] = make_fastdiv((unsigned)R);
+    len /= R;
   }
   return true;
 }
 
-bool make_plan(int N, FftPlan &pl) { return make_plan_order(N, pl, 0); }
+bool make_plan(int N, FftPlan &pl) {
+  pl.div_n = make_fastdiv((unsigned)N);
+  return largest_prime(N) <= 7 && make_plan_order(N, pl, 0);
+}
 
 bool plan_line(int N, FftPlan &pl, int order) {
   const float2 *chirp = pl.chirp, *chirp_ft = pl.chirp_ft;  // tables built by the caller
+  const unsigned short *posof = pl.posof;
   pl.m = 0;
+  if (N > KWB_BLUESTEIN_MAX_N && largest_prime(N) > 7) return false;
   if (!make_plan_order(N, pl, order)) {
     if (N > KWB_BLUESTEIN_MAX_N) return false;
-    int M = 1;
-    while (M < 2 * N - 1) M *= 2;
-    if (!make_plan_order(M, pl, order)) return false;
+    // the inner length: at least 2N - 1, the cheapest by points times stages (a stage costs about
+    // what the loads and stores of a pass do together: two more)
+    int best = 0;
+    long long cost = 0;
+    for (int M = 2 * N - 1; M <= std::min(4 * N, KWB_MAX_N); ++M) {
+      if (!make_plan_order(M, pl, 0)) continue;
+      const long long c = (long long)M * (pl.nstages + 2);
+      if (!best || c < cost) {
+        best = M;
+        cost = c;
+      }
+    }
+    if (!best || !make_plan_order(best, pl, order)) return false;
     pl.n = N;
-    pl.m = M;
+    pl.m = best;
   }
+  pl.div_n = make_fastdiv((unsigned)N);
   pl.chirp = chirp;
   pl.chirp_ft = chirp_ft;
+  pl.posof = posof;
   return true;
 }
 
-// Bluestein tables of an n-point line with inner length m (FP64, rounded once): the chirp
-// w_j = exp(-i pi j^2/n) (j^2 reduced mod 2n exactly, in integers) and FFT_m of its conjugate
-// wrapped to length m (b_j = b_{m-j} = conj(w_j), j < n), scaled by 1/m.
-void bluestein_tables(int n, int m, std::vector<float2> &chirp, std::vector<float2> &chirp_ft) {
+namespace {
+
+using cplx = std::complex<double>;
+
+// out = FFT of n points in[0], in[stride], ... (recursive mixed radix); w: the roots of unity
+// exp(-2 pi i j/N) of the whole transform, of which this one uses every wstep-th.
+void host_fft(const cplx *in, int stride, cplx *out, int n, const std::vector<cplx> &w, int wstep) {
+  if (n == 1) {
+    out[0] = in[0];
+    return;
+  }
+  int p = 2;
+  while (n % p) ++p;
+  const int m = n / p, N = (int)w.size();
+  for (int q = 0; q < p; ++q) host_fft(in + (size_t)q * stride, stride * p, out + (size_t)q * m, m, w, wstep * p);
+  std::vector<cplx> t(p);
+  for (int k = 0; k < m; ++k) {
+    for (int j = 0; j < p; ++j) t[j] = out[(size_t)j * m + k] * w[(size_t)j * k * wstep % N];
+    for (int q = 0; q < p; ++q) {
+      cplx a = 0.0;
+      for (int j = 0; j < p; ++j) a += t[j] * w[(size_t)j * q % p * m * wstep % N];
+      out[(size_t)q * m + k] = a;
+    }
+  }
+}
+
+// FFT_m(in) / m in a plan's digit-reversed order, rounded once to FP32.
+std::vector<float2> spectrum_dif(const std::vector<cplx> &in, const FftPlan &pl) {
   const double pi = 3.141592653589793238462643;
-  std::vector<double> wr(n), wi(n);
+  const int m = (int)in.size();
+  std::vector<cplx> w(m), out(m);
+  for (int j = 0; j < m; ++j) w[j] = cplx(std::cos(2.0 * pi * j / m), -std::sin(2.0 * pi * j / m));
+  host_fft(in.data(), 1, out.data(), m, w, 1);
+  std::vector<float2> f(m);
+  for (int pos = 0; pos < m; ++pos) {
+    int rest = pos, k = 0, wt = 1;
+    for (int s = 0; s < pl.nstages; ++s) {
+      const int q = rest / pl.stride[s];
+      rest -= q * pl.stride[s];
+      k += q * wt;
+      wt *= pl.radix[s];
+    }
+    f[pos] = make_float2((float)(out[k].real() / m), (float)(out[k].imag() / m));
+  }
+  return f;
+}
+
+}  // namespace
+
+// Bluestein tables of an n-point line with the inner transforms of pl (FP64, rounded once): the
+// chirp w_j = exp(-i pi j^2/n) (j^2 reduced mod 2n exactly, in integers) and FFT_m of its conjugate
+// wrapped to length m (b_j = b_{m-j} = conj(w_j), j < n), scaled by 1/m.
+void bluestein_tables(const FftPlan &pl, std::vector<float2> &chirp, std::vector<float2> &chirp_ft) {
+  const double pi = 3.141592653589793238462643;
+  const int n = pl.n, m = pl.m;
+  std::vector<cplx> b(m, 0.0);
+  chirp.resize(n);
   for (int j = 0; j < n; ++j) {
     const long long q = ((long long)j * j) % (2LL * n);
     const double th = pi * (double)q / (double)n;
-    wr[j] = std::cos(th);
-    wi[j] = -std::sin(th);
+    const cplx w(std::cos(th), -std::sin(th));
+    chirp[j] = make_float2((float)w.real(), (float)w.imag());
+    b[j] = std::conj(w);
+    if (j > 0) b[m - j] = std::conj(w);
   }
-  std::vector<double> br(m, 0.0), bi(m, 0.0);
-  for (int j = 0; j < n; ++j) {
-    br[j] = wr[j];
-    bi[j] = -wi[j];
-    if (j > 0) {
-      br[m - j] = wr[j];
-      bi[m - j] = -wi[j];
-    }
-  }
-  // iterative radix-2 FFT (forward, exp(-2 pi i jk/m)), m a power of two
-  for (int i = 1, j = 0; i < m; ++i) {
-    int bit = m >> 1;
-    for (; j & bit; bit >>= 1) j ^= bit;
-    j ^= bit;
-    if (i < j) {
-      std::swap(br[i], br[j]);
-      std::swap(bi[i], bi[j]);
-    }
-  }
-  for (int len = 2; len <= m; len <<= 1) {
-    for (int k = 0; k < len / 2; ++k) {
-      const double a = -2.0 * pi * (double)k / (double)len;
-      const double cr = std::cos(a), ci = std::sin(a);
-      for (int i = 0; i < m; i += len) {
-        const int u = i + k, v = i + k + len / 2;
-        const double tr = br[v] * cr - bi[v] * ci, ti = br[v] * ci + bi[v] * cr;
-        br[v] = br[u] - tr;
-        bi[v] = bi[u] - ti;
-        br[u] += tr;
-        bi[u] += ti;
-      }
-    }
-  }
-  chirp.resize(n);
-  chirp_ft.resize(m);
-  for (int j = 0; j < n; ++j) chirp[j] = make_float2((float)wr[j], (float)wi[j]);
-  for (int k = 0; k < m; ++k) chirp_ft[k] = make_float2((float)(br[k] / m), (float)(bi[k] / m));
+  chirp_ft = spectrum_dif(b, pl);
 }
 
-int choose_L(int N, int want, int cap_lines, int dispersion, bool spec) {
+// Gradient of an n-point line as a convolution of length m (plan pl, m >= 2n - 1): the real kernel
+// h_j = (1/n) sum_k i k_k e^{+-i k_k d/2} e^{2 pi i jk/n} (the multiplier is Hermitian), placed at
+// j and, for negative lags, m + j - n; its FFT_m / m.  sign: +1 or -1 (the half-cell shift).
+std::vector<float2> gradient_conv(const FftPlan &pl, double d, int sign) {
+  const double pi = 3.141592653589793238462643;
+  const int n = pl.n, m = pl.m;
+  std::vector<double> h(n, 0.0);
+  std::vector<cplx> w(2 * n);  // exp(i pi j/n)
+  for (int j = 0; j < 2 * n; ++j) w[j] = cplx(std::cos(pi * j / n), std::sin(pi * j / n));
+  for (int k = 0; k < n; ++k) {
+    const int ks = k < (n + 1) / 2 ? k : k - n;
+    const double kv = 2.0 * pi * ks / (n * d);
+    // k (2 j +- 1) pi / n
+    for (int j = 0; j < n; ++j) {
+      const long long q = ((long long)ks * (2 * j + sign)) % (2 * n);
+      h[j] -= kv * w[q < 0 ? q + 2 * n : q].imag();
+    }
+  }
+  std::vector<cplx> hk(m, 0.0);
+  for (int j = 0; j < n; ++j) {
+    hk[j] = h[j] / n;
+    if (j > 0) hk[m + j - n] = h[j] / n;
+  }
+  return spectrum_dif(hk, pl);
+}
+
+int choose_L(int N, int want, int cap_lines) {
   int L = want;
   if (L < 1) L = 1;
-  while (L > 1 && (spec ? spec_pass_smem(N, L, dispersion) : line_pass_smem(N, L)) > 200 * 1024)
-    L /= 2;
+  while (L > 1 && line_pass_smem(N, L) > 200 * 1024) L /= 2;
   if (cap_lines > 0 && L > cap_lines) L = cap_lines;
   if (L < 1) L = 1;
   return L;
@@ -371,6 +461,8 @@ struct kwb_sim {
   cudaGraphExec_t graph = nullptr;
   int graph_K = 0;
   int launches_per_step = 0;
+  bool steps1d = false;  // whole runs of steps in one launch (launch_steps1d)
+  Groups1D groups1d{};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   ~kwb_sim() {
     if (graph) cudaGraphExecDestroy(graph);
@@ -656,6 +748,7 @@ cudaError_t enqueue_step(kwb_sim *S, long long step_s) {
 }
 
 int count_launches(const kwb_sim *S) {
+  if (S->steps1d) return 1;
   if (S->h.elastic) {
     int n = 2 * S->h.ndim + 2 + (S->h.n_u > 0 ? 1 : 0) + (S->h.n_s > 0 ? 1 : 0);
     for (auto &g : S->groups)
@@ -695,7 +788,7 @@ size_t estimate_device_bytes(const kwb_problem *P) {
     need += (size_t)P->n_s_index * 8 + (size_t)P->n_u_index * 8;
   } else {
     need = (size_t)nvox * 4 * (1 + 2 * D) + (size_t)nspec * 8;
-    if (dispersion) need += (size_t)nvox * 4 + (size_t)nspec * 8;
+    if (dispersion) need += (size_t)nspec * 8;
     need += (size_t)nspec * 4 * (dispersion ? 2 : 1);
     need += (size_t)nvox * 4 * ((r_arr ? 1 : 0) + (c_arr ? 1 : 0) + ((nonlinear && (b_arr || r_arr)) ? 1 : 0));
     // FP64 staging during set-up (released once the simulation is created)
@@ -904,7 +997,6 @@ static int choose_schedule(kwb_sim *S, SimDev &h, cudaStream_t st) {
     if (f) CU(cudaMemsetAsync(f, 0, nvox * 4, st));
   if (h.spec) CU(cudaMemsetAsync(h.spec, 0, h.nspec * sizeof(float2), st));
   if (h.spec2) CU(cudaMemsetAsync(h.spec2, 0, h.nspec * sizeof(float2), st));
-  if (h.rho_prev) CU(cudaMemsetAsync(h.rho_prev, 0, nvox * 4, st));
   schedule_of(h, sc);
   if (pick >= 0) {
     S->schedule_src = "pick " + std::to_string(pick);
@@ -1039,10 +1131,10 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   for (int a = 0; a < 3; ++a) plan_line(h.N[a], h.plan[a], 0);
   int FL[3];  // transform length per axis (the Bluestein inner length where there is one)
   for (int a = 0; a < 3; ++a) FL[a] = fft_len(h.plan[a]);
-  h.L_line[0] = choose_L(FL[0], std::max(1, 2048 / h.N[0]), (h.N[1] + 1) / 2, 0, false);
-  for (int a = 1; a < 3; ++a) h.L_line[a] = choose_L(FL[a], 8, (h.N[0] + 1) / 2, 0, false);
-  h.L_eosx = choose_L(FL[0], std::max(1, 2048 / h.N[0]), (h.N[1] + 1) / 2, h.dispersion, true);
-  for (int a = 1; a < 3; ++a) h.L_spec[a] = choose_L(FL[a], 8, h.n1, h.dispersion, true);
+  h.L_line[0] = choose_L(FL[0], std::max(1, 2048 / h.N[0]), (h.N[1] + 1) / 2);
+  for (int a = 1; a < 3; ++a) h.L_line[a] = choose_L(FL[a], 8, (h.N[0] + 1) / 2);
+  h.L_eosx = choose_L(FL[0], std::max(1, 2048 / h.N[0]), (h.N[1] + 1) / 2);
+  for (int a = 1; a < 3; ++a) h.L_spec[a] = choose_L(FL[a], 8, h.n1);
   h.L_spec[0] = 1;
   {
     // A simulation that runs alone gets narrower tiles and larger CTAs on small grids (latency:
@@ -1118,9 +1210,8 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
     CU(M.alloc(&h.spec, h.nspec));
   }
   if (h.dispersion) {
-    CU(M.alloc(&h.spec2, h.nspec));
-    CU(M.alloc(&h.rho_prev, nvox));
-    CU(cudaMemsetAsync(h.rho_prev, 0, nvox * 4, st));
+    CU(M.alloc(&h.spec2, h.nspec));  // the spectrum of the step before: none yet (rho_prev = 0)
+    CU(cudaMemsetAsync(h.spec2, 0, h.nspec * sizeof(float2), st));
   }
   CU(M.alloc(&S->d_t0, 1));
   CU(cudaMemsetAsync(S->d_t0, 0, 8, st));
@@ -1240,17 +1331,6 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
     CU(M.alloc(&pd, n));
     CU(M.alloc(&psd, n));
     CU(build_twiddles(tw, nt, st));
-    if (h.plan[a].m > 0) {
-      std::vector<float2> ch, chf;
-      bluestein_tables(n, h.plan[a].m, ch, chf);
-      float2 *dch, *dchf;
-      CU(M.alloc(&dch, ch.size()));
-      CU(M.alloc(&dchf, chf.size()));
-      if ((rc = upload(ctx, dch, ch.data(), ch.size() * sizeof(float2), st))) return rc;
-      if ((rc = upload(ctx, dchf, chf.data(), chf.size() * sizeof(float2), st))) return rc;
-      h.plan[a].chirp = dch;
-      h.plan[a].chirp_ft = dchf;
-    }
     const double d = a < D ? P->d[a] : 1.0;
     CU(build_gradient(gp, gn, n, d, st));
     const int psz = a < D ? (int)P->pml_size[a] : 0;
@@ -1270,6 +1350,52 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
       CU(fast_image(n, img, nullptr, tw, gp, gn, psd, pd, st));
       h.img[a] = img;
     }
+  }
+  // Tables in the order of the in-place FFT's stages: the gradients and, with plan.m > 0, the
+  // Bluestein chirp (rebuilt if the schedule takes another radix order).
+  auto stage_tables = [&](int a) -> int {
+    const FftPlan &pl = h.plan[a];
+    const int nt = fft_len(pl);
+    if (pl.m > 0) {
+      std::vector<float2> ch, chf;
+      bluestein_tables(pl, ch, chf);
+      if (int r = upload(ctx, const_cast<float2 *>(pl.chirp), ch.data(), ch.size() * sizeof(float2), st)) return r;
+      if (int r = upload(ctx, const_cast<float2 *>(pl.chirp_ft), chf.data(), chf.size() * sizeof(float2), st)) return r;
+      CU(cudaStreamSynchronize(st));  // the host tables go out of scope
+    }
+    if (pl.posof) CU(build_positions(const_cast<unsigned short *>(pl.posof), pl, st));
+    for (int g = 0; g < 2; ++g) {
+      float2 *out = const_cast<float2 *>(h.gdif[a][g]);
+      if (pl.m > 0) {
+        const std::vector<float2> H = gradient_conv(pl, a < D ? P->d[a] : 1.0, g == 0 ? 1 : -1);
+        if (int r = upload(ctx, out, H.data(), (size_t)nt * sizeof(float2), st)) return r;
+        CU(cudaStreamSynchronize(st));
+      } else {
+        CU(permute_dif(out, g == 0 ? h.gpos[a] : h.gneg[a], pl, st));
+      }
+    }
+    return KWB_OK;
+  };
+  for (int a = 0; a < D; ++a) {
+    const int nt = fft_len(h.plan[a]);
+    for (int g = 0; g < 2; ++g) {
+      float2 *t;
+      CU(M.alloc(&t, nt));
+      h.gdif[a][g] = t;
+    }
+    if (h.plan[a].m == 0) {
+      unsigned short *ps;
+      CU(M.alloc(&ps, nt));
+      h.plan[a].posof = ps;
+    }
+    if (h.plan[a].m > 0) {
+      float2 *ch, *chf;
+      CU(M.alloc(&ch, h.N[a]));
+      CU(M.alloc(&chf, nt));
+      h.plan[a].chirp = ch;
+      h.plan[a].chirp_ft = chf;
+    }
+    if ((rc = stage_tables(a))) return rc;
   }
   if (P->axisymmetric) {
     // 1/r on the radial axis: r = |y_vec|, y_vec = ((0:Ny-1) - (Ny-1)/2) dy, r = 0 -> dy/2
@@ -1293,7 +1419,7 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
     // the x line pass carries the EOS x R2C when both run on the register-FFT kernels
     // (KWB_FUSE_XEOS=0 keeps them separate)
     const char *fx = getenv("KWB_FUSE_XEOS");
-    h.fuse_xeos = (h.fast & 3) == 3 && D >= 2 && !h.dispersion && fast_size(h.N[0]) && !(fx && strcmp(fx, "0") == 0);
+    h.fuse_xeos = (h.fast & 3) == 3 && D >= 2 && fast_size(h.N[0]) && !(fx && strcmp(fx, "0") == 0);
   }
   // The EOS multiplier: allocated here, built once the FFT schedule is known, since the plane
   // pass's slot-major variants read it in their own layout (the tuner's timing launches only
@@ -1434,7 +1560,7 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   // (every voxel) and one sparse group (through a per-x-line index of its points).
   const unsigned ponly = (1u << KWB_REC_P) | (1u << KWB_REC_P_MAX) | (1u << KWB_REC_P_MIN) |
                          (1u << KWB_REC_P_RMS) | (1u << KWB_REC_P_FINAL);
-  const bool fast_inv = (h.fast & 2) && h.ndim >= 2 && !h.dispersion && fast_size(h.N[0]);
+  const bool fast_inv = (h.fast & 2) && h.ndim >= 2 && fast_size(h.N[0]);
   bool sparse_taken = false;
   for (int g = 0; g < P->n_groups; ++g) {
     GroupHost &G = S->groups[g];
@@ -1568,9 +1694,11 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   slog.mark("tr+dense");
   // ---- FFT schedule: measured on first use of this shape (simulations of the batching
   // scheduler share the GPU with others, so they keep the heuristic)
-  if (!ctx->batched && S->Nt_loop > 0) {
+  if (!ctx->batched && S->Nt_loop > 0 && (P->progress || !steps1d_fits(h))) {
     if ((rc = choose_schedule(S.get(), h, st))) return rc;
     CU(h.elastic ? el_prime(h) : prime_attributes(h));
+    for (int a = 0; a < D; ++a)
+      if (h.plan_order[a] != 0 && (rc = stage_tables(a))) return rc;
   }
   if (!h.elastic) {
     // [kz][ky][kx]; with the plane pass [kx][kz][slot], or [kx][slot][k_z in register order]
@@ -1579,6 +1707,16 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
     CU(build_eos_multiplier(const_cast<float *>(h.M), const_cast<float *>(h.M2), h.N, d3, c_ref, P->dt,
                             c_arr ? 1.0 : c_s * c_s, absorbing, tau, eta, y, h.plane ? slot_ky : nullptr,
                             fast_plane_slot_major(h) ? slot_kz : nullptr, st));
+  }
+
+  if (D == 1 && steps1d_fits(h)) {
+    const int n = h.N[0];
+    float2 *nat, *op;
+    CU(M.alloc(&nat, n));
+    CU(M.alloc(&op, n));
+    CU(build_eos1d(nat, h.M, n, st));
+    CU(permute_dif(op, nat, h.plan[0], st));
+    h.eos1d = op;
   }
 
   slog.mark("schedule");
@@ -1602,6 +1740,20 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   S->progress = P->progress;
   S->progress_user = P->progress_user;
   if (S->progress) CU(cudaMallocHost(&S->p_host, nvox * 4));
+  if (!S->progress && steps1d_fits(h)) {
+    Groups1D &g1 = S->groups1d;
+    int live = 0;
+    for (auto &G : S->groups) {
+      if (G.spec.cartesian || G.n == 0) continue;
+      if (live < KWB_1D_GROUPS) g1.g[live] = G.d_dev;
+      ++live;
+    }
+    g1.n = live;
+    if (live <= KWB_1D_GROUPS) {
+      CU(steps1d_prime(h));
+      S->steps1d = true;
+    }
+  }
   S->launches_per_step = count_launches(S.get());
   slog.done();
   *out = S.release();
@@ -1622,6 +1774,15 @@ static int sim_enqueue(kwb_sim *S, long long steps) {
       CU(cudaStreamSynchronize(S->stream));
       S->steps_done++;
       S->progress(t + 1, S->Nt_loop, S->p_host, S->progress_user);
+    }
+    return KWB_OK;
+  }
+  if (S->steps1d) {
+    while (steps > 0) {  // launches of a millisecond or two
+      const int k = (int)std::min<long long>(steps, 16 * KWB_CHUNK_STEPS);
+      CU(launch_steps1d(S->h, S->groups1d, S->steps_done, k, S->stream));
+      S->steps_done += k;
+      steps -= k;
     }
     return KWB_OK;
   }
@@ -1672,7 +1833,7 @@ int kwb_sim_advance_timed(kwb_sim *S, int64_t steps, double *device_ms) {
   kwb_ctx *ctx = S->ctx;
   CU(cudaSetDevice(ctx->device));
   // capture the replayed chunk first, so that the timed interval holds device work only
-  if (!S->progress && !S->graph && steps >= KWB_CHUNK_STEPS && S->Nt_loop - S->steps_done >= KWB_CHUNK_STEPS) {
+  if (!S->progress && !S->steps1d && !S->graph && steps >= KWB_CHUNK_STEPS && S->Nt_loop - S->steps_done >= KWB_CHUNK_STEPS) {
     const int rc = build_chunk_graph(S);
     if (rc) return rc;
   }
@@ -1994,7 +2155,7 @@ int kwb_sim_profile(kwb_sim *S, int64_t steps, kwb_kernel_times *out) {
       continue;
     }
     if (S->tr) timed(slot("tr_inject", h.n_tr * 8.0), [&] { return launch_tr_inject(S->d_sim, h, s, st); });
-    const double eos_rd = nv * 4.0 * (h.D + (h.c0sq ? 1 : 0) + (h.nonlinear && h.nlq ? 1 : 0) + (h.dispersion ? 2 : 0));
+    const double eos_rd = nv * 4.0 * (h.D + (h.c0sq ? 1 : 0) + (h.nonlinear && h.nlq ? 1 : 0));
     for (int a : {1, 2, 0}) {
       if (a >= h.ndim) continue;
       static const char *nm[3] = {"line_pass_x", "line_pass_y", "line_pass_z"};
@@ -2004,15 +2165,15 @@ int kwb_sim_profile(kwb_sim *S, int64_t steps, kwb_kernel_times *out) {
             [&] { return launch_line_pass(S->d_sim, h, a, KWB_MODE_STEP, s, st); });
     }
     if (!h.fuse_xeos)
-      timed(slot("eos_x_fwd", eos_rd + ns * 8.0 * (h.dispersion ? 2 : 1)), [&] { return launch_eos_x_fwd(S->d_sim, h, s, st); });
+      timed(slot("eos_x_fwd", eos_rd + ns * 8.0), [&] { return launch_eos_x_fwd(S->d_sim, h, s, st); });
     if (h.ndim == 2) {
-      timed(slot("spec_y_mul", ns * 8.0 * (h.dispersion ? 3 : 2) + ns * 4.0 * (h.dispersion ? 2 : 1)),
+      timed(slot("spec_y_mul", ns * 8.0 * (h.dispersion ? 4 : 2) + ns * 4.0 * (h.dispersion ? 2 : 1)),
             [&] { return launch_spec_pass(S->d_sim, h, 1, KWB_SPEC_FWD_MUL_INV, s, st); });
     } else if (h.ndim == 3 && h.plane) {
       timed(slot("spec_yz_plane", ns * 16.0 + ns * 4.0), [&] { return fast_plane(S->d_sim, h, s, st); });
     } else if (h.ndim == 3) {
-      timed(slot("spec_y_fwd", ns * 16.0 * (h.dispersion ? 2 : 1)), [&] { return launch_spec_pass(S->d_sim, h, 1, KWB_SPEC_FWD, s, st); });
-      timed(slot("spec_z_mul", ns * 8.0 * (h.dispersion ? 3 : 2) + ns * 4.0 * (h.dispersion ? 2 : 1)),
+      timed(slot("spec_y_fwd", ns * 16.0), [&] { return launch_spec_pass(S->d_sim, h, 1, KWB_SPEC_FWD, s, st); });
+      timed(slot("spec_z_mul", ns * 8.0 * (h.dispersion ? 4 : 2) + ns * 4.0 * (h.dispersion ? 2 : 1)),
             [&] { return launch_spec_pass(S->d_sim, h, 2, KWB_SPEC_FWD_MUL_INV, s, st); });
       timed(slot("spec_y_inv", ns * 16.0), [&] { return launch_spec_pass(S->d_sim, h, 1, KWB_SPEC_INV, s, st); });
     }

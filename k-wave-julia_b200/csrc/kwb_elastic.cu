@@ -20,7 +20,7 @@
 // Each directional derivative is the 1-D transform along its axis (the reference's full N-D
 // rfft / irfft with a multiplier that varies along one axis only), computed two real lines per
 // complex line: power-of-two lines on the register FFTs of kwb_fast.cu (k_el_grad_fast), other
-// lengths on the shared-memory Stockham FFTs of kwb_fft.cuh (k_el_grad below).
+// lengths on the in-place FFTs of kwb_generic.cu (k_el_grad).
 #include <algorithm>
 
 #include "kwb_fft.cuh"
@@ -47,76 +47,6 @@ __device__ __forceinline__ Coord coord_of(const SimDev &S, long long i) {
 }
 
 }  // namespace
-
-// Directional derivatives of g.nf fields along `axis` on one tile of 2L real lines.
-template <bool CONTIG>
-__global__ void __launch_bounds__(KWB_PASS_THREADS_MAX)
-    k_el_grad(const __grid_constant__ SimDev S, int axis, const __grid_constant__ ElGrad g, long long step_s) {
-  extern __shared__ float4 smem_raw[];
-  const int N = S.N[axis];
-  const int L = S.L_line[axis];
-  const int LS = line_pitch(fft_len(S.plan[axis]));
-  const int Nx = S.N[0];
-  float2 *X = reinterpret_cast<float2 *>(smem_raw);
-  float2 *Y = X + L * LS;
-  float2 *tw = Y + L * LS;
-  load_twiddles(tw, S.tw[axis], fft_len(S.plan[axis]));  // set-up-time table: before waiting on the previous kernel
-  KWB_STEP_KERNEL_PROLOGUE();
-  if (step_index(S, step_s) >= S.Nt) return;
-  const Tile T = CONTIG ? tile_x(S, 2 * L, blockIdx.x) : tile_yz(S, axis, 2 * L, blockIdx.x);
-  auto addr = [&](int c, int i) -> long long {
-    return CONTIG ? T.base + (long long)c * Nx + i : T.base + (long long)i * T.stride + c;
-  };
-  // element e of the tile: line l, position i (strided tiles keep neighbouring columns adjacent
-  // in a warp, so their global accesses coalesce)
-  auto decode = [&](int e, int &l, int &i) {
-    if (CONTIG) {
-      l = e / N;
-      i = e - l * N;
-    } else {
-      i = e / L;
-      l = e - i * L;
-    }
-  };
-  const int total = L * N;
-  const float2 *__restrict__ mult = g.neg ? S.gneg[axis] : S.gpos[axis];
-  for (int f = 0; f < g.nf; ++f) {
-    const float *__restrict__ src = g.src[f];
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      int l, i;
-      decode(e, l, i);
-      const int ca = 2 * l, cb = 2 * l + 1;
-      const float a = ca < T.cnt ? src[addr(ca, i)] : 0.f;
-      const float b = cb < T.cnt ? src[addr(cb, i)] : 0.f;
-      X[l * LS + i] = make_float2(a, b);
-    }
-    __syncthreads();
-    float2 *R = fft_lines<false>(X, Y, L, LS, S.plan[axis], tw);
-    float2 *F = (R == X) ? Y : X;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      const int l = e / N, i = e - l * N;
-      R[l * LS + i] = cmul(R[l * LS + i], mult[i]);  // i k e^{+-i k d/2} / N
-    }
-    __syncthreads();
-    const float2 *Dv = fft_lines<true>(R, F, L, LS, S.plan[axis], tw);
-    float *dst = g.dst[f];
-    const bool acc = (g.acc >> f) & 1;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      int l, i;
-      decode(e, l, i);
-      const float2 d = Dv[l * LS + i];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = 2 * l + h;
-        if (c >= T.cnt) continue;
-        const long long ad = addr(c, i);
-        const float dv = h ? d.y : d.x;
-        dst[ad] = acc ? dst[ad] + dv : dv;
-      }
-    }
-    __syncthreads();  // X and Y are refilled by the next field
-  }
-}
 
 // v_j = pml_sg,j (pml_sg,j v_j + dt / rho_sg,j w_j), pml = 1 - deficit; rho_sg,j the periodic
 // average of rho0 with its +1 neighbour along j (_stagger_density_{2,3}d, first_order_steps.jl:
@@ -368,19 +298,14 @@ static int elementwise_grid(const SimDev &h) {
   return (int)std::max(1LL, std::min(want, cap));
 }
 
-static cudaError_t set_smem_optin(const void *fn, size_t bytes) { return raise_dynamic_smem(fn, bytes); }
-
-// Register-FFT passes serve power-of-two lines (strided ones need Nx a multiple of 4 for their
-// 16-byte staging); every other length runs on the Stockham kernel above.
+// Register-FFT passes serve the lengths of kwb_fast.cu (strided ones need Nx a multiple of 4 for
+// their 16-byte staging); every other length runs on the in-place FFTs (kwb_generic.cu).
 static bool el_fast(const SimDev &h, int axis) {
   return (h.fast & 1) && fast_size(h.N[axis]) && (axis == 0 || h.N[0] % 4 == 0);
 }
 
 cudaError_t el_prime(const SimDev &h) {
-  cudaError_t e = set_smem_optin((const void *)k_el_grad<true>, line_pass_smem(fft_len(h.plan[0]), h.L_line[0]));
-  size_t m = 0;
-  for (int a = 1; a < h.ndim; ++a) m = std::max(m, line_pass_smem(fft_len(h.plan[a]), h.L_line[a]));
-  if (e == cudaSuccess) e = set_smem_optin((const void *)k_el_grad<false>, m);
+  cudaError_t e = generic_el_prime(h);
   for (int a = 0; a < h.ndim && e == cudaSuccess; ++a)
     if (el_fast(h, a)) e = fast_prime(h.N[a]);
   return e;
@@ -388,16 +313,7 @@ cudaError_t el_prime(const SimDev &h) {
 
 cudaError_t el_grad(const SimDev &h, int axis, const ElGrad &g, long long s, cudaStream_t st) {
   if (el_fast(h, axis)) return fast_el_grad(h, axis, g, s, st);
-  const int L = h.L_line[axis];
-  const size_t sm = line_pass_smem(fft_len(h.plan[axis]), L);
-  const long long tiles = axis == 0 ? (long long)cdiv(h.N[1], 2 * L) * h.N[2]
-                                    : (long long)cdiv(h.N[0], 2 * L) * (axis == 1 ? h.N[2] : h.N[1]);
-  const int threads = pass_threads(h, tiles, (long long)L * h.N[axis]);
-  if (axis == 0)
-    kwb_launch(k_el_grad<true>, (int)tiles, threads, sm, st, h, axis, g, s);
-  else
-    kwb_launch(k_el_grad<false>, (int)tiles, threads, sm, st, h, axis, g, s);
-  return cudaGetLastError();
+  return generic_el_grad(h, axis, g, s, st);
 }
 
 static bool vec4(const SimDev &h) { return h.N[0] % 4 == 0 && h.nvox < (1LL << 31); }

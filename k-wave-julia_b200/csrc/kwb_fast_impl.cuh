@@ -10,7 +10,7 @@
 // (coalesced across threads) and prefetched ahead of the transform arithmetic.
 //
 // Same semantics as the generic shared-memory Stockham kernels (kwb_kernels.cu), which keep
-// serving every other line length (radix 3/5/7 sizes) and the :stokes dispersion branch.
+// serving every other line length.
 #pragma once
 #include <algorithm>
 
@@ -176,7 +176,7 @@ __device__ __forceinline__ void dft_mixed(float2 (&v)[E]) {
   if constexpr ((E & (E - 1)) == 0) {
     dft_reg<E, INV>(v);
   } else if constexpr (E == 3 || E == 5) {
-    Dft<E, INV>::run(v);
+    dft_any<E, INV>(v);
   } else {
     constexpr int P = (E % 3 == 0) ? 3 : 5;
     constexpr int Q = E / P;
@@ -187,7 +187,7 @@ __device__ __forceinline__ void dft_mixed(float2 (&v)[E]) {
       float2 w[P];
 #pragma unroll
       for (int n1 = 0; n1 < P; ++n1) w[n1] = v[Q * n1 + n2];
-      Dft<P, INV>::run(w);
+      dft_any<P, INV>(w);
 #pragma unroll
       for (int k1 = 0; k1 < P; ++k1) a[n2 * P + k1] = rotE<E, INV>(w[k1], n2 * k1);
     }
@@ -1652,7 +1652,20 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
       return;
     }
 #pragma unroll
-    for (int idx = 0; idx < E; ++idx) v[idx] = cscale(v[idx], m[idx]);
+    for (int idx = 0; idx < E; ++idx) {
+      if (!S.dispersion) {
+        v[idx] = cscale(v[idx], m[idx]);
+        continue;
+      }
+      // dispersion: this pass keeps each step's spectrum for the next (build_eos_multiplier)
+      const int k = F::k_of(tt, idx);
+      const long long mi = (axis == 1) ? ((long long)o * Ny + k) * n1 + k0 + l
+                                       : ((long long)k * Ny + o) * n1 + k0 + l;
+      const float m2 = valid ? __ldg(S.M2 + mi) : 0.f;
+      const float2 b = valid ? __ldcg(S.spec2 + mi) : make_float2(0.f, 0.f);
+      if (valid) S.spec2[mi] = v[idx];
+      v[idx] = pfma(pair(m2), b, pmul(pair(m[idx]), v[idx]));
+    }
     F::inv(v, xs, tw2, tt);
   }
   if (valid) {

@@ -1,15 +1,10 @@
-// Batched mixed-radix (2, 3, 4, 5, 7, 8) Stockham FFTs in shared memory.
+// Register DFTs of any radix up to 16, and the small arithmetic the transform kernels share.
 //
-// A CTA holds L complex lines of length N, line stride LS, in shared memory and transforms all
-// of them at once: every stage is one pass of radix-R butterflies over L*N/R butterflies
-// shared by the CTA's threads, ping-ponging between two buffers.  The Stockham ordering keeps
-// the output in natural frequency order, so the k-space multiplies index it directly.
-//
-// Twiddles exp(-2 pi i m / N) come from a table built in FP64 on the device and rounded once
-// to FP32 (kwb_tables.cu); the butterfly constants are the exact values of cos/sin(2 pi k/R)
-// written out to 22 digits.  Forward = exp(-i...), inverse = exp(+i...) without 1/N (the
-// normalisation is folded into the k-space multipliers).
+// The in-place shared-memory transforms for any line length are in kwb_generic.cu, the
+// register-resident ones for the lengths they cover in kwb_fast_impl.cuh.
 #pragma once
+#include <type_traits>
+
 #include "kwb_internal.h"
 
 namespace kwb {
@@ -17,9 +12,12 @@ namespace kwb {
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+// (packed FP32 pairs: per component the round-to-nearest result of the scalar operation, in one
+// instruction for both)
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
+__device__ __forceinline__ float2 cfma(float s, float2 a, float2 b) { return __ffma2_rn(make_float2(s, s), a, b); }
 // multiply by -i (forward) or +i (inverse)
 template <bool INV>
 __device__ __forceinline__ float2 mul_mi(float2 a) {
@@ -51,230 +49,150 @@ struct Dft<4, INV> {
   }
 };
 
-template <bool INV>
-struct Dft<8, INV> {
-  __device__ __forceinline__ static void run(float2 (&v)[8]) {
-    const float h = 0.7071067811865475244008f;
-    float2 e[4] = {v[0], v[2], v[4], v[6]};
-    float2 o[4] = {v[1], v[3], v[5], v[7]};
-    Dft<4, INV>::run(e);
-    Dft<4, INV>::run(o);
-    // W^1 = (1 -+ i)/sqrt2, W^2 = -+i, W^3 = (-1 -+ i)/sqrt2
-    float2 w1 = INV ? make_float2(h * (o[1].x - o[1].y), h * (o[1].x + o[1].y))
-                    : make_float2(h * (o[1].x + o[1].y), h * (o[1].y - o[1].x));
-    float2 w2 = mul_mi<INV>(o[2]);
-    float2 w3 = INV ? make_float2(-h * (o[3].x + o[3].y), h * (o[3].x - o[3].y))
-                    : make_float2(h * (o[3].y - o[3].x), -h * (o[3].x + o[3].y));
-    v[0] = cadd(e[0], o[0]);
-    v[4] = csub(e[0], o[0]);
-    v[1] = cadd(e[1], w1);
-    v[5] = csub(e[1], w1);
-    v[2] = cadd(e[2], w2);
-    v[6] = csub(e[2], w2);
-    v[3] = cadd(e[3], w3);
-    v[7] = csub(e[3], w3);
-  }
-};
+// ---- register DFTs of any radix up to 16
 
-template <bool INV>
-struct Dft<3, INV> {
-  __device__ __forceinline__ static void run(float2 (&v)[3]) {
-    const float s3 = 0.8660254037844386467637f;
-    float2 t = cadd(v[1], v[2]);
-    float2 s = mul_mi<INV>(cscale(csub(v[1], v[2]), s3));
-    float2 m = make_float2(fmaf(-0.5f, t.x, v[0].x), fmaf(-0.5f, t.y, v[0].y));
-    v[0] = cadd(v[0], t);
-    v[1] = cadd(m, s);
-    v[2] = csub(m, s);
-  }
+// cos and sin of 2 pi m / R, m < R, in double by their Taylor series after folding into [0, pi/4]
+// (evaluated at compile time, rounded once to FP32).
+struct CosSin {
+  double c, s;
 };
-
-template <bool INV>
-struct Dft<5, INV> {
-  __device__ __forceinline__ static void run(float2 (&v)[5]) {
-    const float c1 = 0.3090169943749474241023f, c2 = -0.8090169943749474241023f;
-    const float s1 = 0.9510565162951535721164f, s2 = 0.5877852522924731291687f;
-    float2 t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
-    float2 t3 = csub(v[1], v[4]), t4 = csub(v[2], v[3]);
-    float2 a1 = make_float2(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
-    float2 a2 = make_float2(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-    float2 b1 = mul_mi<INV>(make_float2(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y));
-    float2 b2 = mul_mi<INV>(make_float2(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y));
-    v[0] = cadd(v[0], cadd(t1, t2));
-    v[1] = cadd(a1, b1);
-    v[4] = csub(a1, b1);
-    v[2] = cadd(a2, b2);
-    v[3] = csub(a2, b2);
+__host__ __device__ constexpr CosSin cos_sin_turn(int m, int R) {
+  // m/R of a turn; fold by symmetry to the first octant, in integers (eighths of a turn: 8 m / R)
+  bool neg_s = false, neg_c = false, swap = false;
+  if (2 * m > R) {
+    m = R - m;
+    neg_s = true;
   }
+  // now 0 <= m/R <= 1/2
+  int num = m, den = R;  // angle = num/den turns
+  if (4 * num > den) {   // second quadrant: pi - x
+    num = den - 2 * num;
+    den = 2 * den;
+    neg_c = true;
+  }
+  if (8 * num > den) {  // beyond pi/4: pi/2 - x
+    num = den - 4 * num;
+    den = 4 * den;
+    swap = true;
+  }
+  const double x = 6.283185307179586476925286766559 * num / den;
+  double c = 0.0, s = 0.0, t = 1.0;
+  for (int k = 0; k < 24; ++k) {
+    const double v = ((k / 2) % 2 == 0) ? t : -t;
+    if (k % 2 == 0) c += v;
+    else s += v;
+    t = t * x / (k + 1);
+  }
+  const double cc = swap ? s : c, ss = swap ? c : s;
+  return CosSin{neg_c ? -cc : cc, neg_s ? -ss : ss};
+}
+// (value and the remainder of its rounding to FP32: the constants of a radix act on every butterfly
+// alike, so an error in one is a gain, the same on every step, that adds up over a simulation --
+// 5e-8 a convolution at N = 100, 1e-5 over 200 steps -- where the roundings of the arithmetic average
+// out)
+template <int R>
+struct Roots {
+  float c[R], s[R], cl[R], sl[R];
 };
+template <int R>
+__host__ __device__ constexpr Roots<R> make_roots() {
+  Roots<R> r{};
+  for (int m = 0; m < R; ++m) {
+    const CosSin v = cos_sin_turn(m, R);
+    r.c[m] = (float)v.c;
+    r.s[m] = (float)v.s;
+    r.cl[m] = (float)(v.c - (double)r.c[m]);
+    r.sl[m] = (float)(v.s - (double)r.s[m]);
+  }
+  return r;
+}
 
-template <bool INV>
-struct Dft<7, INV> {
-  __device__ __forceinline__ static void run(float2 (&v)[7]) {
-    const float c[3] = {0.6234898018587335305251f, -0.2225209339563144042889f,
-                        -0.9009688679024191262361f};
-    const float s[3] = {0.7818314824680298087084f, 0.9749279121818236070181f,
-                        0.4338837391175581204758f};
-    float2 t[3], d[3];
+// v exp(-+ 2 pi i m / R) for a compile-time m
+template <int R, bool INV>
+__device__ __forceinline__ float2 root_mul(float2 v, int m) {
+  constexpr Roots<R> W = make_roots<R>();
+  m %= R;
+  if (m == 0) return v;
+  if (4 * m == R) return mul_mi<INV>(v);
+  if (2 * m == R) return make_float2(-v.x, -v.y);
+  if (4 * m == 3 * R) return mul_mi<!INV>(v);
+  const float c = W.c[m], s = INV ? -W.s[m] : W.s[m];
+  const float cl = W.cl[m], sl = INV ? -W.sl[m] : W.sl[m];
+  return make_float2(fmaf(v.x, c, fmaf(v.y, s, fmaf(v.x, cl, v.y * sl))),
+                     fmaf(v.y, c, fmaf(-v.x, s, fmaf(v.y, cl, -v.x * sl))));
+}
+
+__host__ __device__ constexpr int first_factor(int R) {
+  return R % 4 == 0 && R > 4 ? 4 : R % 3 == 0 && R > 3 ? 3 : R % 2 == 0 && R > 2 ? 2 : R;
+}
+// R-point DFT in registers, natural order in and out: R = 1, 2, 4, an odd prime (pairs v_j +-
+// v_{R-j}), or one Cooley-Tukey step P * Q (n = Q n1 + n2, k = k1 + P k2).
+template <int R, bool INV>
+__device__ __forceinline__ void dft_any(float2 (&v)[R]) {
+  constexpr int P = first_factor(R);
+  if constexpr (R == 1) {
+    return;
+  } else if constexpr (R == 2 || R == 4) {
+    Dft<R, INV>::run(v);
+  } else if constexpr (P == R) {
+    constexpr Roots<R> W = make_roots<R>();
+    constexpr int H = (R - 1) / 2;
+    float2 t[H], d[H];
+    float2 sum = v[0];
+    const float2 x0 = v[0];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      t[j] = cadd(v[j + 1], v[6 - j]);
-      d[j] = csub(v[j + 1], v[6 - j]);
+    for (int j = 0; j < H; ++j) {
+      t[j] = cadd(v[j + 1], v[R - 1 - j]);
+      d[j] = csub(v[j + 1], v[R - 1 - j]);
+      sum = cadd(sum, t[j]);
     }
-    float2 x0 = v[0];
-    v[0] = cadd(x0, cadd(t[0], cadd(t[1], t[2])));
+    v[0] = sum;
 #pragma unroll
-    for (int k = 1; k <= 3; ++k) {
-      float2 a = x0, b = make_float2(0.f, 0.f);
+    for (int k = 1; k <= H; ++k) {
+      float2 a = make_float2(0.f, 0.f), b = a;
 #pragma unroll
-      for (int j = 1; j <= 3; ++j) {
-        int m = (j * k) % 7;  // cos(2 pi m/7), sin(2 pi m/7) with m in 1..6
-        float cm = m <= 3 ? c[m - 1] : c[7 - m - 1];
-        float sm = m <= 3 ? s[m - 1] : -s[7 - m - 1];
-        a.x = fmaf(cm, t[j - 1].x, a.x);
-        a.y = fmaf(cm, t[j - 1].y, a.y);
-        b.x = fmaf(sm, d[j - 1].x, b.x);
-        b.y = fmaf(sm, d[j - 1].y, b.y);
+      for (int j = 1; j <= H; ++j) {  // the remainders first: the small terms
+        const float c = W.cl[(j * k) % R], s = W.sl[(j * k) % R];
+        a = cfma(c, t[j - 1], a);
+        b = cfma(s, d[j - 1], b);
       }
+#pragma unroll
+      for (int j = 1; j <= H; ++j) {
+        const float c = W.c[(j * k) % R], s = W.s[(j * k) % R];
+        a = cfma(c, t[j - 1], a);
+        b = cfma(s, d[j - 1], b);
+      }
+      a = cadd(a, x0);
       b = mul_mi<INV>(b);
       v[k] = cadd(a, b);
-      v[7 - k] = csub(a, b);
+      v[R - k] = csub(a, b);
+    }
+  } else {
+    constexpr int Q = R / P;
+    float2 a[R];
+#pragma unroll
+    for (int n2 = 0; n2 < Q; ++n2) {
+      float2 w[P];
+#pragma unroll
+      for (int n1 = 0; n1 < P; ++n1) w[n1] = v[Q * n1 + n2];
+      dft_any<P, INV>(w);
+#pragma unroll
+      for (int k1 = 0; k1 < P; ++k1) a[n2 * P + k1] = root_mul<R, INV>(w[k1], n2 * k1);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < P; ++k1) {
+      float2 w[Q];
+#pragma unroll
+      for (int n2 = 0; n2 < Q; ++n2) w[n2] = a[n2 * P + k1];
+      dft_any<Q, INV>(w);
+#pragma unroll
+      for (int k2 = 0; k2 < Q; ++k2) v[k1 + P * k2] = w[k2];
     }
   }
-};
-
-// Line pitch (float2 slots per line) of the Stockham buffers: N elements plus one pad slot per 16
-// for the intermediate stages (see spad), plus one.
-__host__ __device__ inline int line_pitch(int N) { return N + (N >> 4) + 1; }
-
-// Slot of element m in an intermediate stage buffer: one pad slot after every 16 elements, so
-// the strided stores of the early stages (stride R * Ns with Ns < 16) fall in distinct banks.
-// The first stage reads, and the last stage writes, the natural (unpadded) order the callers
-// use.
-__device__ __forceinline__ int spad(int m) { return m + (m >> 4); }
+}
 
 __device__ __forceinline__ int fdiv(int n, FastDiv d) {
   return (int)((__umulhi((unsigned)n, d.mul) + (unsigned)n) >> d.shift);
-}
-
-// One Stockham stage of radix R over L lines: X -> Y (pin / pout: X / Y in the padded layout).
-// dnr, dns: divisions by N / R and by Ns, precomputed in the plan.
-template <int R, bool INV>
-__device__ __forceinline__ void stockham_stage(const float2 *__restrict__ X, float2 *__restrict__ Y,
-                                               int L, int LS, int N, int Ns,
-                                               const float2 *__restrict__ tw, bool pin, bool pout,
-                                               FastDiv dnr, FastDiv dns) {
-  const int NR = N / R;
-  const int total = L * NR;
-  const int tstride = N / (Ns * R);
-  for (int b = threadIdx.x; b < total; b += blockDim.x) {
-    const int l = fdiv(b, dnr);
-    const int j = b - l * NR;
-    const int k = j - fdiv(j, dns) * Ns;
-    const float2 *x = X + l * LS;
-    float2 *y = Y + l * LS;
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int m = j + r * NR;
-      v[r] = x[pin ? spad(m) : m];
-    }
-    if (k != 0) {
-      const int ts = k * tstride;
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        float2 w = tw[r * ts];
-        if (INV) w.y = -w.y;
-        v[r] = cmul(v[r], w);
-      }
-    }
-    Dft<R, INV>::run(v);
-    const int base = (j - k) * R + k;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int m = base + r * Ns;
-      y[pout ? spad(m) : m] = v[r];
-    }
-  }
-}
-
-// The Stockham stages of `plan` on L lines of fft_len(plan) points held in X (Y is scratch).
-template <bool INV>
-__device__ float2 *stockham_lines(float2 *X, float2 *Y, int L, int LS, const FftPlan &plan,
-                                  const float2 *tw) {
-  const int N = fft_len(plan);
-  int Ns = 1;
-  for (int s = 0; s < plan.nstages; ++s) {
-    const int R = plan.radix[s];
-    const bool pin = s > 0, pout = s + 1 < plan.nstages;
-    const FastDiv dnr = plan.div_nr[s], dns = plan.div_ns[s];
-    switch (R) {
-      case 2: stockham_stage<2, INV>(X, Y, L, LS, N, Ns, tw, pin, pout, dnr, dns); break;
-      case 3: stockham_stage<3, INV>(X, Y, L, LS, N, Ns, tw, pin, pout, dnr, dns); break;
-      case 4: stockham_stage<4, INV>(X, Y, L, LS, N, Ns, tw, pin, pout, dnr, dns); break;
-      case 5: stockham_stage<5, INV>(X, Y, L, LS, N, Ns, tw, pin, pout, dnr, dns); break;
-      case 7: stockham_stage<7, INV>(X, Y, L, LS, N, Ns, tw, pin, pout, dnr, dns); break;
-      default: stockham_stage<8, INV>(X, Y, L, LS, N, Ns, tw, pin, pout, dnr, dns); break;
-    }
-    __syncthreads();
-    float2 *t = X;
-    X = Y;
-    Y = t;
-    Ns *= R;
-  }
-  return X;
-}
-
-// Bluestein's algorithm for the n-point DFT of L lines (n = plan.n, first n slots of each line
-// in X; X and Y hold plan.m slots per line): with w_j = exp(-i pi j^2/n),
-//   X_k = w_k sum_j (x_j w_j) conj(w_{k-j}),
-// a circular convolution of length m >= 2n - 1 done as FFT_m, a multiply by the transform of
-// the conjugate chirp (chirp_ft, scaled by 1/m), and an inverse FFT_m.  The inverse DFT is the
-// conjugate of the forward DFT of the conjugate input.  tw: the m-point twiddles.
-template <bool INV>
-__device__ float2 *bluestein_lines(float2 *X, float2 *Y, int L, int LS, const FftPlan &plan,
-                                   const float2 *tw) {
-  const int n = plan.n, m = plan.m;
-  const float2 *__restrict__ w = plan.chirp;
-  const float2 *__restrict__ B = plan.chirp_ft;
-  for (int e = threadIdx.x; e < L * m; e += blockDim.x) {
-    const int l = e / m, j = e - l * m;
-    float2 a = make_float2(0.f, 0.f);
-    if (j < n) {
-      float2 x = X[l * LS + j];
-      if (INV) x.y = -x.y;
-      a = cmul(x, w[j]);
-    }
-    Y[l * LS + j] = a;
-  }
-  __syncthreads();
-  float2 *R = stockham_lines<false>(Y, X, L, LS, plan, tw);
-  float2 *F = (R == Y) ? X : Y;
-  for (int e = threadIdx.x; e < L * m; e += blockDim.x) {
-    const int l = e / m, j = e - l * m;
-    R[l * LS + j] = cmul(R[l * LS + j], B[j]);
-  }
-  __syncthreads();
-  float2 *C = stockham_lines<true>(R, F, L, LS, plan, tw);
-  for (int e = threadIdx.x; e < L * n; e += blockDim.x) {
-    const int l = e / n, k = e - l * n;
-    float2 v = cmul(C[l * LS + k], w[k]);
-    if (INV) v.y = -v.y;
-    C[l * LS + k] = v;
-  }
-  __syncthreads();
-  return C;
-}
-
-// Transform L lines held in X (Y is scratch of the same size; line pitch
-// LS >= line_pitch(fft_len(plan))).  Returns the buffer holding the result (X or Y), the first
-// plan.n slots of each line in natural order.  Caller must __syncthreads() before (X filled) --
-// this function syncs after every stage, so the result is visible to all threads on return.
-template <bool INV>
-__device__ float2 *fft_lines(float2 *X, float2 *Y, int L, int LS, const FftPlan &plan,
-                             const float2 *tw) {
-  if (plan.m > 0) return bluestein_lines<INV>(X, Y, L, LS, plan, tw);
-  return stockham_lines<INV>(X, Y, L, LS, plan, tw);
 }
 
 }  // namespace kwb

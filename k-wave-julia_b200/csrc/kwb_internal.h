@@ -16,9 +16,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#define KWB_MAX_STAGES 16
+#define KWB_MAX_STAGES 8
 #define KWB_THREADS 256
-#define KWB_PASS_THREADS_MAX 1024  // Stockham passes on grids with few tiles (pass_threads)
+#define KWB_PASS_THREADS_MAX 256  // threads per CTA of the passes on the in-place FFTs (pass_threads)
 #define KWB_MAX_N 4096
 #define KWB_BLUESTEIN_MAX_N 2048  // Bluestein inner length 4096 at most: one line fits shared memory
 #define KWB_CHUNK_STEPS 32  // time steps per replayed CUDA graph
@@ -35,10 +35,13 @@
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); \
   } while (0)
 
-// Stockham plan of a line of n points.  A length with a prime factor above 7 is transformed by
-// Bluestein's algorithm (chirp z-transform): m > 0 is the power-of-two length of the inner
-// transforms (m >= 2n - 1), the stages are m's, chirp[j] = exp(-i pi j^2 / n) (j < n) and
-// chirp_ft = FFT_m(conj chirp, wrapped) / m; m == 0 for a direct transform.
+// In-place FFT plan of a line of n points (kwb_generic.cu): radices of the forward stages, first to
+// last (1, then N, for a length of one stage, so that there are always two or more).  A length with
+// a prime factor above 13 has m > 0: its line passes run the gradient, a circular convolution of
+// length n, as one of length m >= 2n - 1 without wrap-around (m small-radix; the gradient tables
+// hold the kernel's transform), and its equation-of-state passes run Bluestein's algorithm (chirp
+// z-transform) with inner transforms of m points, chirp[j] = exp(-i pi j^2 / n) (j < n) and chirp_ft
+// = FFT_m(conj chirp, wrapped) / m in the stages' order.  m == 0: direct transforms of n points.
 // Division by a run-time constant d as a multiply and shift: n / d == (umulhi(n, mul) + n) >> shift
 // for 0 <= n < 2^31 (mul = floor(2^32 (2^shift - d) / d) + 1, shift = ceil(log2 d)).
 struct FastDiv {
@@ -57,10 +60,15 @@ struct FftPlan {
   int m;
   const float2 *chirp;
   const float2 *chirp_ft;
-  // per stage: division by the butterflies per line (len / radix) and by the sub-transform
-  // length so far (the product of the earlier radices)
-  FastDiv div_nr[KWB_MAX_STAGES];
-  FastDiv div_ns[KWB_MAX_STAGES];
+  const unsigned short *posof;  // digit-reversed position of each frequency (nullptr: worked out)
+  FastDiv div_n;  // division by n
+  // per stage: butterflies per line, positions between a butterfly's elements, twiddle-table step,
+  // and the divisions by the stride and by the radix
+  int nbf[KWB_MAX_STAGES];
+  int stride[KWB_MAX_STAGES];
+  int tstride[KWB_MAX_STAGES];
+  FastDiv div_st[KWB_MAX_STAGES];
+  FastDiv div_r[KWB_MAX_STAGES];
 };
 // Length of the transforms a plan runs (the buffers and twiddle table of a line are this long).
 __host__ __device__ inline int fft_len(const FftPlan &p) { return p.m > 0 ? p.m : p.n; }
@@ -98,9 +106,8 @@ struct SimDev {
   float *p;
   float *u[3];
   float *rho[3];
-  float *rho_prev;  // dispersion only
   float2 *spec;
-  float2 *spec2;    // dispersion only
+  float2 *spec2;    // dispersion only: the spectrum of rho_eff at the last step, kept by the pass that multiplies
 
   const float *rho0;  // nullptr: scalar density
   const float *c0sq;  // nullptr: scalar sound speed
@@ -108,15 +115,19 @@ struct SimDev {
   const float *nlq;   // nullptr: scalar Q (nlq_s)
   float nlq_s;
   int nonlinear;
-  int dispersion;     // scalar c0 with :stokes absorption -> second spectrum
+  int dispersion;     // scalar c0 with :stokes absorption -> M2 and spec2
   int scalar_c;       // c^2 folded into M (scalar c0) vs applied per voxel
   const float *M;     // [Nz][Ny][n1]; plane pass: [n1][Nz][slot] or slot-major [n1][slot][z]
-  const float *M2;    // dispersion multiplier, [Nz][Ny][n1]
+  const float *M2;    // dispersion: multiplier of the last step's spectrum, [Nz][Ny][n1]
 
   const float *pml_def[3];
   const float *pml_sg_def[3];
   const float2 *gpos[3];
   const float2 *gneg[3];
+  // the gradient operators of the in-place FFT's line passes, in its digit-reversed order: staggered
+  // + (0) and - (1); with plan.m > 0 the transforms of the gradient's convolution kernels
+  const float2 *gdif[3][2];
+  const float2 *eos1d;  // 1-D: the equation of state's full-length operator in that order
   const float2 *tw[3];
   const float2 *img[3];  // table image of each register-FFT axis (fast_image), nullptr otherwise
   FftPlan plan[3];
@@ -258,21 +269,40 @@ namespace kwb {
 // Let kernel fn take `bytes` of dynamic shared memory: raises its limit to the device's opt-in
 // maximum less the kernel's own static shared memory (cudaErrorInvalidValue if bytes exceed it).
 cudaError_t raise_dynamic_smem(const void *fn, size_t bytes);
-// Stockham plan of a line of N points (false: a prime factor above 7 or too many stages), and
-// the complex lines per tile of a line pass (spec = false) or spectrum pass (spec = true) that
-// fit the shared-memory budget, at most cap_lines (kwb_api.cu).
+// Stages of a transform of N points (false: a prime factor above 13), radices in ascending order;
+// order 1: radices of one prime, or 4; order 2: as 0 in descending order.  make_plan also refuses
+// prime factors above 7 (callers that cannot take the tables the longer ones may need).
 bool make_plan(int N, FftPlan &pl);
-// The same stages in another order: 0 as make_plan (8s first, then 4 or 2, then 3, 5, 7),
-// 1 radix-4 stages instead of 8s, 2 the odd radices first.
 bool make_plan_order(int N, FftPlan &pl, int order);
-// The plan of a line of N points: direct Stockham stages when N is 2/3/5/7-smooth, else
-// Bluestein with a power-of-two inner length (N <= KWB_BLUESTEIN_MAX_N); keeps pl's chirp tables.
+// The plan of a line of N points: direct stages, or m > 0 (N <= KWB_BLUESTEIN_MAX_N); keeps pl's
+// chirp tables.
 bool plan_line(int N, FftPlan &pl, int order);
-int choose_L(int N, int want, int cap_lines, int dispersion, bool spec);
+// Complex lines per tile of a pass that fit the shared-memory budget, at most cap_lines (kwb_api.cu).
+int choose_L(int N, int want, int cap_lines);
 size_t line_pass_smem(int N, int L);
-size_t spec_pass_smem(int N, int L, int dispersion);
-// threads per CTA of a Stockham line pass along `axis` (-1: not a line pass)
-int pass_threads(const SimDev &h, long long tiles, long long elems_per_tile, int axis = -1);
+// The passes on the in-place FFTs (kwb_generic.cu); the primes raise their kernels' shared memory.
+struct ElGrad;
+cudaError_t generic_prime(const SimDev &h);
+cudaError_t generic_line_pass(const SimDev &h, int axis, int mode, long long step_s, cudaStream_t st);
+cudaError_t generic_eos(const SimDev &h, bool fwd, long long step_s, cudaStream_t st);
+cudaError_t generic_spec(const SimDev &h, int axis, int op, long long step_s, cudaStream_t st);
+cudaError_t generic_el_prime(const SimDev &h);
+cudaError_t generic_el_grad(const SimDev &h, int axis, const ElGrad &g, long long s, cudaStream_t st);
+// lines of a position side by side in shared memory: an odd pitch, or a multiple of 8
+__host__ __device__ inline int lines_pitch(int L) { return L % 8 == 0 ? L : L | 1; }
+// 1-D simulations: `steps` time steps from step t_first in one launch (kwb_generic.cu), for direct
+// transforms whose state fits shared memory and at most KWB_1D_GROUPS recorded sensor groups.
+#define KWB_1D_GROUPS 8
+struct Groups1D {
+  int n;
+  const GroupDev *g[KWB_1D_GROUPS];
+};
+bool steps1d_fits(const SimDev &h);
+cudaError_t steps1d_prime(const SimDev &h);
+cudaError_t build_eos1d(float2 *out, const float *M, int N, cudaStream_t st);
+cudaError_t launch_steps1d(const SimDev &h, const Groups1D &g, long long t_first, int steps, cudaStream_t st);
+// threads per CTA of a pass of L lines on the in-place FFTs (tuned > 0: that many)
+int pass_threads(const FftPlan &pl, int L, int tuned);
 cudaError_t launch_line_pass(const SimDev *d_sim, const SimDev &h, int axis, int mode,
                              long long step_s, cudaStream_t st);
 cudaError_t launch_eos_x_fwd(const SimDev *d_sim, const SimDev &h, long long step_s,
@@ -448,6 +478,9 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
 
 // FP64 table builders.
 cudaError_t build_twiddles(float2 *out, int N, cudaStream_t st);
+// out[position] = in[frequency] in the digit-reversed order of a plan
+cudaError_t permute_dif(float2 *out, const float2 *in, const FftPlan &pl, cudaStream_t st);
+cudaError_t build_positions(unsigned short *posof, const FftPlan &pl, cudaStream_t st);
 cudaError_t build_gradient(float2 *pos, float2 *neg, int N, double d, cudaStream_t st);
 cudaError_t build_pml_deficit(float *out, int N, int pml_size, double alpha, double dt,
                               int staggered, cudaStream_t st);

@@ -87,8 +87,16 @@ __global__ void k_build_eos_multiplier(float *M, float *M2, int Nx, int Ny, int 
   const double inv_total = 1.0 / ((double)Nx * (double)Ny * (double)Nz);
   double m = c_sq_fold * kappa;
   if (absorbing) m = m * (1.0 + tau * pow(kmag, y));
-  M[idx] = (float)(m * inv_total);
-  if (M2) M2[idx] = (float)(c_sq_fold * kappa * (eta * pow(kmag, y - 1.0)) * inv_total);
+  // Dispersion (first_order_steps.jl:255-263): M F - M2 (F - F_prev)/dt with F, F_prev the spectra of
+  // rho_eff at this step and the last. The transform being linear, F_prev is the last step's
+  // spectrum itself, kept by the pass that multiplies: M then holds M - M2/dt, and M2 holds M2/dt.
+  if (M2) {
+    const double m2 = c_sq_fold * kappa * (eta * pow(kmag, y - 1.0)) * inv_total / dt;
+    M[idx] = (float)(m * inv_total - m2);
+    M2[idx] = (float)m2;
+  } else {
+    M[idx] = (float)(m * inv_total);
+  }
 }
 
 // Row-major (x slowest, f fastest: in[(x*Nm + m)*Nf + f]) to column-major
@@ -146,6 +154,30 @@ cudaError_t build_twiddles(float2 *out, int N, cudaStream_t st) {
   k_build_twiddles<<<blocks(N, 256), 256, 0, st>>>(out, N);
   return cudaGetLastError();
 }
+static __global__ void k_permute_dif(float2 *out, const float2 *in, unsigned short *posof,
+                                     const __grid_constant__ FftPlan pl) {
+  const int N = fft_len(pl);
+  for (int pos = blockIdx.x * blockDim.x + threadIdx.x; pos < N; pos += gridDim.x * blockDim.x) {
+    int rest = pos, k = 0, w = 1;
+    for (int s = 0; s < pl.nstages; ++s) {
+      const int q = rest / pl.stride[s];
+      rest -= q * pl.stride[s];
+      k += q * w;
+      w *= pl.radix[s];
+    }
+    if (out) out[pos] = in[k];
+    else posof[k] = (unsigned short)pos;
+  }
+}
+cudaError_t build_positions(unsigned short *posof, const FftPlan &pl, cudaStream_t st) {
+  k_permute_dif<<<(fft_len(pl) + 255) / 256, 256, 0, st>>>(nullptr, nullptr, posof, pl);
+  return cudaGetLastError();
+}
+cudaError_t permute_dif(float2 *out, const float2 *in, const FftPlan &pl, cudaStream_t st) {
+  k_permute_dif<<<(fft_len(pl) + 255) / 256, 256, 0, st>>>(out, in, nullptr, pl);
+  return cudaGetLastError();
+}
+
 cudaError_t build_gradient(float2 *pos, float2 *neg, int N, double d, cudaStream_t st) {
   k_build_gradient<<<blocks(N, 256), 256, 0, st>>>(pos, neg, N, d);
   return cudaGetLastError();

@@ -58,8 +58,17 @@ __device__ __forceinline__ long long step_index(const SimDev &S, long long step_
   return *S.t0 + step_s;
 }
 
+// Asynchronous copy of N twiddles into shared memory (8 bytes each: the table follows the line
+// buffer, whose size is any multiple of 8); twiddles_landed() before their first use.
 __device__ __forceinline__ void load_twiddles(float2 *tw, const float2 *g, int N) {
-  for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = g[i];
+  for (int i = threadIdx.x; i < N; i += blockDim.x)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(tw + i)),
+                 "l"(g + i)
+                 : "memory");
+}
+__device__ __forceinline__ void twiddles_landed() {
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
 }
 
 }  // namespace kwb
