@@ -89,118 +89,14 @@ __device__ __forceinline__ void dft_reg(float2 (&v)[E]) {
   for (int q = 0; q < E; ++q) v[q] = t[q];
 }
 
-// cos(2 pi j/120) and sin(2 pi j/120), j = 0..119: the roots of unity of the 12- and 20-point
-// register DFTs (exact values to 18 significant digits)
-__device__ constexpr float kCos120[120] = {
-    1.00000000000000000e+00f, 9.98629534754573833e-01f, 9.94521895368273290e-01f, 9.87688340595137770e-01f,
-    9.78147600733805689e-01f, 9.65925826289068312e-01f, 9.51056516295153531e-01f, 9.33580426497201743e-01f,
-    9.13545457642600867e-01f, 8.91006524188367899e-01f, 8.66025403784438708e-01f, 8.38670567945424050e-01f,
-    8.09016994374947451e-01f, 7.77145961456970902e-01f, 7.43144825477394244e-01f, 7.07106781186547573e-01f,
-    6.69130606358858238e-01f, 6.29320391049837502e-01f, 5.87785252292473137e-01f, 5.44639035015027195e-01f,
-    5.00000000000000000e-01f, 4.53990499739546804e-01f, 4.06736643075800375e-01f, 3.58367949545300379e-01f,
-    3.09016994374947451e-01f, 2.58819045102520739e-01f, 2.07911690817759232e-01f, 1.56434465040230924e-01f,
-    1.04528463267653457e-01f, 5.23359562429437444e-02f, 0.00000000000000000e+00f, -5.23359562429436195e-02f,
-    -1.04528463267653332e-01f, -1.56434465040230813e-01f, -2.07911690817759343e-01f, -2.58819045102520628e-01f,
-    -3.09016994374947340e-01f, -3.58367949545300268e-01f, -4.06736643075800042e-01f, -4.53990499739546693e-01f,
-    -5.00000000000000000e-01f, -5.44639035015026751e-01f, -5.87785252292473026e-01f, -6.29320391049837280e-01f,
-    -6.69130606358857905e-01f, -7.07106781186547462e-01f, -7.43144825477394022e-01f, -7.77145961456970902e-01f,
-    -8.09016994374947340e-01f, -8.38670567945423939e-01f, -8.66025403784438708e-01f, -8.91006524188367788e-01f,
-    -9.13545457642600978e-01f, -9.33580426497201743e-01f, -9.51056516295153531e-01f, -9.65925826289068312e-01f,
-    -9.78147600733805689e-01f, -9.87688340595137659e-01f, -9.94521895368273401e-01f, -9.98629534754573833e-01f,
-    -1.00000000000000000e+00f, -9.98629534754573833e-01f, -9.94521895368273401e-01f, -9.87688340595137770e-01f,
-    -9.78147600733805689e-01f, -9.65925826289068423e-01f, -9.51056516295153642e-01f, -9.33580426497201854e-01f,
-    -9.13545457642600867e-01f, -8.91006524188367899e-01f, -8.66025403784438819e-01f, -8.38670567945424050e-01f,
-    -8.09016994374947562e-01f, -7.77145961456971013e-01f, -7.43144825477394244e-01f, -7.07106781186547684e-01f,
-    -6.69130606358858460e-01f, -6.29320391049837835e-01f, -5.87785252292473248e-01f, -5.44639035015026973e-01f,
-    -5.00000000000000000e-01f, -4.53990499739546916e-01f, -4.06736643075800874e-01f, -3.58367949545299880e-01f,
-    -3.09016994374947562e-01f, -2.58819045102520628e-01f, -2.07911690817759787e-01f, -1.56434465040231035e-01f,
-    -1.04528463267654234e-01f, -5.23359562429434252e-02f, 0.00000000000000000e+00f, 5.23359562429439457e-02f,
-    1.04528463267652985e-01f, 1.56434465040230675e-01f, 2.07911690817759426e-01f, 2.58819045102521128e-01f,
-    3.09016994374947229e-01f, 3.58367949545299547e-01f, 4.06736643075799764e-01f, 4.53990499739546638e-01f,
-    5.00000000000000000e-01f, 5.44639035015026640e-01f, 5.87785252292472915e-01f, 6.29320391049836836e-01f,
-    6.69130606358858460e-01f, 7.07106781186547351e-01f, 7.43144825477394244e-01f, 7.77145961456970569e-01f,
-    8.09016994374947340e-01f, 8.38670567945423606e-01f, 8.66025403784438819e-01f, 8.91006524188367788e-01f,
-    9.13545457642600978e-01f, 9.33580426497201521e-01f, 9.51056516295153531e-01f, 9.65925826289068312e-01f,
-    9.78147600733805689e-01f, 9.87688340595137659e-01f, 9.94521895368273290e-01f, 9.98629534754573833e-01f};
-__device__ constexpr float kSin120[120] = {
-    0.00000000000000000e+00f, 5.23359562429438277e-02f, 1.04528463267653457e-01f, 1.56434465040230869e-01f,
-    2.07911690817759315e-01f, 2.58819045102520739e-01f, 3.09016994374947396e-01f, 3.58367949545300268e-01f,
-    4.06736643075800153e-01f, 4.53990499739546749e-01f, 5.00000000000000000e-01f, 5.44639035015026973e-01f,
-    5.87785252292473137e-01f, 6.29320391049837502e-01f, 6.69130606358858238e-01f, 7.07106781186547462e-01f,
-    7.43144825477394133e-01f, 7.77145961456970902e-01f, 8.09016994374947451e-01f, 8.38670567945423939e-01f,
-    8.66025403784438597e-01f, 8.91006524188367788e-01f, 9.13545457642600867e-01f, 9.33580426497201743e-01f,
-    9.51056516295153531e-01f, 9.65925826289068312e-01f, 9.78147600733805689e-01f, 9.87688340595137770e-01f,
-    9.94521895368273290e-01f, 9.98629534754573833e-01f, 1.00000000000000000e+00f, 9.98629534754573833e-01f,
-    9.94521895368273401e-01f, 9.87688340595137770e-01f, 9.78147600733805689e-01f, 9.65925826289068312e-01f,
-    9.51056516295153642e-01f, 9.33580426497201743e-01f, 9.13545457642600978e-01f, 8.91006524188367899e-01f,
-    8.66025403784438708e-01f, 8.38670567945424272e-01f, 8.09016994374947451e-01f, 7.77145961456971013e-01f,
-    7.43144825477394466e-01f, 7.07106781186547573e-01f, 6.69130606358858349e-01f, 6.29320391049837391e-01f,
-    5.87785252292473248e-01f, 5.44639035015027306e-01f, 5.00000000000000000e-01f, 4.53990499739546860e-01f,
-    4.06736643075800042e-01f, 3.58367949545300213e-01f, 3.09016994374947507e-01f, 2.58819045102520573e-01f,
-    2.07911690817759315e-01f, 1.56434465040230980e-01f, 1.04528463267653290e-01f, 5.23359562429438069e-02f,
-    0.00000000000000000e+00f, -5.23359562429435640e-02f, -1.04528463267653055e-01f, -1.56434465040230730e-01f,
-    -2.07911690817759065e-01f, -2.58819045102520351e-01f, -3.09016994374947285e-01f, -3.58367949545299991e-01f,
-    -4.06736643075800208e-01f, -4.53990499739546693e-01f, -5.00000000000000000e-01f, -5.44639035015027084e-01f,
-    -5.87785252292473026e-01f, -6.29320391049837169e-01f, -6.69130606358858238e-01f, -7.07106781186547462e-01f,
-    -7.43144825477394022e-01f, -7.77145961456970569e-01f, -8.09016994374947340e-01f, -8.38670567945424050e-01f,
-    -8.66025403784438375e-01f, -8.91006524188367788e-01f, -9.13545457642600534e-01f, -9.33580426497201854e-01f,
-    -9.51056516295153531e-01f, -9.65925826289068312e-01f, -9.78147600733805578e-01f, -9.87688340595137659e-01f,
-    -9.94521895368273290e-01f, -9.98629534754573944e-01f, -1.00000000000000000e+00f, -9.98629534754573833e-01f,
-    -9.94521895368273401e-01f, -9.87688340595137770e-01f, -9.78147600733805578e-01f, -9.65925826289068201e-01f,
-    -9.51056516295153642e-01f, -9.33580426497202076e-01f, -9.13545457642601089e-01f, -8.91006524188368010e-01f,
-    -8.66025403784438597e-01f, -8.38670567945424272e-01f, -8.09016994374947562e-01f, -7.77145961456971346e-01f,
-    -7.43144825477394022e-01f, -7.07106781186547684e-01f, -6.69130606358858127e-01f, -6.29320391049837835e-01f,
-    -5.87785252292473359e-01f, -5.44639035015027750e-01f, -5.00000000000000000e-01f, -4.53990499739546971e-01f,
-    -4.06736643075800153e-01f, -3.58367949545300768e-01f, -3.09016994374947618e-01f, -2.58819045102520684e-01f,
-    -2.07911690817758982e-01f, -1.56434465040231119e-01f, -1.04528463267653415e-01f, -5.23359562429443689e-02f};
-
-// x * exp(-+2 pi i m/E) for compile-time m and E (E divides 120)
-template <int E, bool INV>
-__device__ __forceinline__ float2 rotE(float2 x, int m) {
-  m %= E;
-  if (m == 0) return x;
-  const int j = m * (120 / E);
-  if (j == 30) return mul_mi<INV>(x);
-  if (j == 60) return make_float2(-x.x, -x.y);
-  if (j == 90) return mul_mi<!INV>(x);
-  const float c = kCos120[j];
-  const float s = INV ? -kSin120[j] : kSin120[j];
-  return make_float2(fmaf(x.x, c, x.y * s), fmaf(x.y, c, -x.x * s));
-}
-
-// E-point DFT in registers, natural order in and out, for E = 2^a (dft_reg), 3, 5, or an odd
-// prime P in {3, 5} times a smaller such length Q (one Cooley-Tukey step, n = Q n1 + n2,
-// k = k1 + P k2: P-point DFTs over n1, twiddles exp(-2 pi i n2 k1/E), Q-point DFTs over n2).
+// E-point DFT in registers, natural order in and out: powers of two (dft_reg), and the mixed radices
+// 3 ... 20 with the constants' remainders carried (dft_any): with FP32 constants alone a 1000-point
+// line (20 * 5 * 10) had a gain that brought a 1000^2 solve 1.2e-5 off over 300 steps, against
+// 4e-6 at 256 x 64.
 template <int E, bool INV>
 __device__ __forceinline__ void dft_mixed(float2 (&v)[E]) {
-  if constexpr ((E & (E - 1)) == 0) {
-    dft_reg<E, INV>(v);
-  } else if constexpr (E == 3 || E == 5) {
-    dft_any<E, INV>(v);
-  } else {
-    constexpr int P = (E % 3 == 0) ? 3 : 5;
-    constexpr int Q = E / P;
-    static_assert(P * Q == E && 120 % E == 0, "register DFT length");
-    float2 a[E];
-#pragma unroll
-    for (int n2 = 0; n2 < Q; ++n2) {
-      float2 w[P];
-#pragma unroll
-      for (int n1 = 0; n1 < P; ++n1) w[n1] = v[Q * n1 + n2];
-      dft_any<P, INV>(w);
-#pragma unroll
-      for (int k1 = 0; k1 < P; ++k1) a[n2 * P + k1] = rotE<E, INV>(w[k1], n2 * k1);
-    }
-#pragma unroll
-    for (int k1 = 0; k1 < P; ++k1) {
-      float2 w[Q];
-#pragma unroll
-      for (int n2 = 0; n2 < Q; ++n2) w[n2] = a[n2 * P + k1];
-      dft_mixed<Q, INV>(w);
-#pragma unroll
-      for (int k2 = 0; k2 < Q; ++k2) v[k1 + P * k2] = w[k2];
-    }
-  }
+  if constexpr ((E & (E - 1)) == 0) dft_reg<E, INV>(v);
+  else dft_any<E, INV>(v);
 }
 
 __device__ __forceinline__ float2 cmul_conj(float2 a, float2 w) {  // a * conj(w)
