@@ -251,7 +251,8 @@ int kwb_sim_profile(kwb_sim *sim, int64_t steps, kwb_kernel_times *out);
  * keeps no file).  KWB_TUNE=0 keeps the size heuristic. */
 int kwb_sim_schedule(const kwb_sim *sim, char *buf, int64_t len);
 
-/* Device bytes the simulation holds and kernels launched per time step. */
+/* Device bytes the simulation holds and kernels launched per time step (1 for a 1-D simulation that
+ * runs many steps in one launch). */
 int kwb_sim_info(const kwb_sim *sim, int64_t *device_bytes, int32_t *launches_per_step);
 
 /* Device bytes a simulation of `problem` would hold (what admission compares with free memory). */

@@ -948,7 +948,7 @@ static void sched_store_locked(const std::string &key, const std::string &val) {
 }
 
 // Raised when the step kernels change, so that a file's measurements of older ones are not used.
-#define KWB_SCHED_GEN 2
+#define KWB_SCHED_GEN 3
 
 static std::string sched_key(int device, const SimDev &h) {
   // the device's name, asked once: the query takes 2.5 ms, a sixth of a 128^2 solve of 689 steps
@@ -1164,7 +1164,7 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
     h.grid_fill = !ctx->batched && !(gf && strcmp(gf, "0") == 0);
   }
   if (h.grid_fill) {
-    // Small grids: fewer lines per tile until the shared-memory (Stockham) passes fill the GPU --
+    // Small grids: fewer lines per tile until the in-place passes fill the GPU --
     // a 384^2 grid otherwise runs its x pass as 39 CTAs and its y spectrum pass as 25.  Strided
     // line passes stop at one wave and keep 4 complex lines (8 columns: one 32-byte sector per
     // row), since narrower tiles waste most of each sector they read.

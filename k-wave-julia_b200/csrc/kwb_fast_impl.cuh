@@ -9,8 +9,8 @@
 // the thread that loaded it.  Field operands are loaded straight from HBM into registers
 // (coalesced across threads) and prefetched ahead of the transform arithmetic.
 //
-// Same semantics as the generic shared-memory Stockham kernels (kwb_kernels.cu), which keep
-// serving every other line length.
+// Same semantics as the in-place shared-memory kernels (kwb_generic.cu), which serve every other
+// line length.
 #pragma once
 #include <algorithm>
 
@@ -906,19 +906,26 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   // memory (entry by entry at the point of use, a chain of three loads each, they held the tiles of
   // a 9 x 9 disc source up by 3-4 us a pass).  More than SRC_CAP entries on a tile are read in
   // place.
-  constexpr int SRC_CAP = THREADS < 32 ? THREADS : 32;
+  constexpr int SRC_CAP = 128, SRC_PER = (SRC_CAP + THREADS - 1) / THREADS;
   __shared__ int src_ptr[2][2 * LT + 1];
   __shared__ int2 src_ent[2][SRC_CAP];  // line << 16 | position, value
   const bool has_u = mode == KWB_MODE_STEP && S.u_sig[axis] && S.u_line_ptr[axis];
   const bool has_p = mode == KWB_MODE_STEP && S.n_p > 0 && S.p_line_ptr[axis];
-  int my_j[2] = {-1, -1};
+  int my_j[2][SRC_PER];
+#pragma unroll
+  for (int c = 0; c < SRC_PER; ++c) my_j[0][c] = my_j[1][c] = -1;
   auto src_find = [&](int k, const int *lp, const SrcEntry *en) {
     const int q0 = __ldg(lp + first_line), n = __ldg(lp + first_line + cnt) - q0;
     for (int c = tid; c <= cnt; c += THREADS) src_ptr[k][c] = __ldg(lp + first_line + c) - q0;
-    if (tid < n && n <= SRC_CAP) {
-      const SrcEntry e = en[q0 + tid];
-      src_ent[k][tid].x = (e.line - first_line) << 16 | e.pos;
-      my_j[k] = e.j;
+    if (n > SRC_CAP) return;
+#pragma unroll
+    for (int c = 0; c < SRC_PER; ++c) {
+      const int q = tid + c * THREADS;
+      if (q < n) {
+        const SrcEntry e = en[q0 + q];
+        src_ent[k][q].x = (e.line - first_line) << 16 | e.pos;
+        my_j[k][c] = e.j;
+      }
     }
   };
   if (has_u) src_find(0, S.u_line_ptr[axis], S.u_entry[axis]);
@@ -950,13 +957,16 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     }
   }
   const long long t = *S.t0 + step_s;
-  if (my_j[0] >= 0) {
-    const int tcol = (int)(min(t + 1, (long long)S.u_cols[axis]) - 1);
-    src_ent[0][tid].y = __float_as_int(S.u_sig[axis][(long long)tcol * S.n_u + my_j[0]]);
-  }
-  if (my_j[1] >= 0) {
-    const int tcol = (int)(min(t + 1, (long long)S.p_cols) - 1);
-    src_ent[1][tid].y = __float_as_int(S.p_sig[(long long)tcol * S.n_p + my_j[1]]);
+#pragma unroll
+  for (int c = 0; c < SRC_PER; ++c) {
+    if (my_j[0][c] >= 0) {
+      const int tcol = (int)(min(t + 1, (long long)S.u_cols[axis]) - 1);
+      src_ent[0][tid + c * THREADS].y = __float_as_int(S.u_sig[axis][(long long)tcol * S.n_u + my_j[0][c]]);
+    }
+    if (my_j[1][c] >= 0) {
+      const int tcol = (int)(min(t + 1, (long long)S.p_cols) - 1);
+      src_ent[1][tid + c * THREADS].y = __float_as_int(S.p_sig[(long long)tcol * S.n_p + my_j[1][c]]);
+    }
   }
   float2 *xs = sm + l * LP;
   float *__restrict__ ud = S.u[axis];
@@ -1325,6 +1335,12 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     qb = __ldg(lp + 1);
     qc = vb ? __ldg(lp + 2) : qb;
   }
+  int2 ent_a = make_int2(0, 0), ent_b = ent_a;  // this thread's first point on either row
+  if (tt < qb - qa) ent_a = __ldg(gs->line_ent + qa + tt);
+  if (tt < qc - qb) ent_b = __ldg(gs->line_ent + qb + tt);
+  const unsigned gs_mask = gs ? gs->mask : 0u;
+  const long long gs_n = gs ? gs->n : 0;
+  float *const gs_ser = gs ? gs->ser_p : nullptr;
   pdl_wait();
   const long long t = *S.t0 + step_s;
   // The half spectrum's rows, all of a thread's loads in flight at once (k = tt + G j, and the
@@ -1464,17 +1480,17 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
 #pragma unroll
     for (int r = 0; r < E; ++r) xs[tt + G * r] = v[r];
     F::sync();
-    const unsigned sm_ = gs->mask;
+    const unsigned sm_ = gs_mask;
     const bool last = (t == S.Nt - 1);
     for (int c = 0; c < 2; ++c) {
       if (!(c ? vb : va)) continue;
       const int q0 = c ? qb : qa, q1 = c ? qc : qb;
       for (int q = q0 + tt; q < q1; q += G) {
-        const int2 e = gs->line_ent[q];
+        const int2 e = q - q0 >= G ? gs->line_ent[q] : c ? ent_b : ent_a;
         const float2 pp = xs[e.x];
         const float pv = c ? pp.y : pp.x;
         const long long j = e.y;
-        if (sm_ & (1u << 0)) gs->ser_p[t * gs->n + j] = pv;
+        if (sm_ & (1u << 0)) gs_ser[t * gs_n + j] = pv;
         if (sm_ & (1u << 1)) gs->pmax[j] = fmaxf(gs->pmax[j], pv);
         if (sm_ & (1u << 2)) gs->pmin[j] = fminf(gs->pmin[j], pv);
         if (sm_ & (1u << 3)) gs->prms[j] += (double)gs->cnt_prms * ((double)pv * (double)pv);
@@ -1547,20 +1563,33 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
       }
       return;
     }
+    if (!S.dispersion) {
 #pragma unroll
-    for (int idx = 0; idx < E; ++idx) {
-      if (!S.dispersion) {
-        v[idx] = cscale(v[idx], m[idx]);
-        continue;
+      for (int idx = 0; idx < E; ++idx) v[idx] = cscale(v[idx], m[idx]);
+    } else {
+      // dispersion: this pass keeps each step's spectrum for the next (build_eos_multiplier); a batch
+      // of loads before the first store (one by one they took 14 us of a 384 x 320 pass)
+      constexpr int B4 = 4;
+      static_assert(E % B4 == 0, "batches of four");
+#pragma unroll
+      for (int i0 = 0; i0 < E; i0 += B4) {
+        float m2[B4];
+        float2 b[B4];
+        long long mi[B4];
+#pragma unroll
+        for (int j = 0; j < B4; ++j) {
+          const int k = F::k_of(tt, i0 + j);
+          mi[j] = (axis == 1) ? ((long long)o * Ny + k) * n1 + k0 + l : ((long long)k * Ny + o) * n1 + k0 + l;
+          m2[j] = valid ? __ldg(S.M2 + mi[j]) : 0.f;
+          b[j] = valid ? __ldcg(S.spec2 + mi[j]) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int j = 0; j < B4; ++j) {
+          const int idx = i0 + j;
+          if (valid) S.spec2[mi[j]] = v[idx];
+          v[idx] = pfma(pair(m2[j]), b[j], pmul(pair(m[idx]), v[idx]));
+        }
       }
-      // dispersion: this pass keeps each step's spectrum for the next (build_eos_multiplier)
-      const int k = F::k_of(tt, idx);
-      const long long mi = (axis == 1) ? ((long long)o * Ny + k) * n1 + k0 + l
-                                       : ((long long)k * Ny + o) * n1 + k0 + l;
-      const float m2 = valid ? __ldg(S.M2 + mi) : 0.f;
-      const float2 b = valid ? __ldcg(S.spec2 + mi) : make_float2(0.f, 0.f);
-      if (valid) S.spec2[mi] = v[idx];
-      v[idx] = pfma(pair(m2), b, pmul(pair(m[idx]), v[idx]));
     }
     F::inv(v, xs, tw2, tt);
   }
@@ -1965,6 +1994,19 @@ struct LinePolicy<768> {
   static constexpr int THREADS = 256, MINB = 2;
 };
 
+// CTAs per SM that a tile of LT lines is compiled for: as many threads an SM as the full-width tile's
+// (with its two CTAs for every width, a 128-thread tile of 256 points took 230 registers a thread and
+// ran 2 CTAs, 8 warps, an SM).  The mixed radices, of 12 or 20 elements a thread, need those
+// registers: held to 128, the 160^3 y pass went from 50 to 67 us.
+template <int N>
+constexpr int min_ctas(int LT) {
+  using P = LinePolicy<N>;
+  constexpr int G = P::template F<true>::G;
+  if ((N & (N - 1)) != 0) return P::MINB;
+  const int m = P::MINB * (P::THREADS / G) / LT;
+  return m > 16 ? 16 : m < 1 ? 1 : m;
+}
+
 // elastic gradient pass (defined below), primed with the line-pass variants of the same tiles
 template <class F, bool CONTIG, int LT, int MINB>
 __global__ void __launch_bounds__(LT * F::G, MINB)
@@ -1974,12 +2016,12 @@ template <int N, bool C, int LT>
 static inline cudaError_t prime_line_variant() {
   using P = LinePolicy<N>;
   using F = typename P::template F<C>;
-  cudaError_t e = raise_smem((const void *)k_line_fast<F, C, LT, P::MINB, false>, pline_smem<F>(LT));
-  if (e == cudaSuccess) e = raise_smem((const void *)k_el_grad_fast<F, C, LT, P::MINB>, pline_smem<F>(LT));
+  cudaError_t e = raise_smem((const void *)k_line_fast<F, C, LT, min_ctas<N>(LT), false>, pline_smem<F>(LT));
+  if (e == cudaSuccess) e = raise_smem((const void *)k_el_grad_fast<F, C, LT, min_ctas<N>(LT)>, pline_smem<F>(LT));
   if constexpr (C) {
-    if (e == cudaSuccess) e = raise_smem((const void *)k_line_fast<F, C, LT, P::MINB, true>, pline_smem<F>(LT));
+    if (e == cudaSuccess) e = raise_smem((const void *)k_line_fast<F, C, LT, min_ctas<N>(LT), true>, pline_smem<F>(LT));
   } else {
-    if (e == cudaSuccess) e = raise_smem((const void *)k_line_fast<F, C, LT, P::MINB, false, true>, pline_smem<F>(LT));
+    if (e == cudaSuccess) e = raise_smem((const void *)k_line_fast<F, C, LT, min_ctas<N>(LT), false, true>, pline_smem<F>(LT));
   }
   return e;
 }
@@ -2017,9 +2059,9 @@ static inline void line_go(const SimDev *d_sim, const SimDev &h, int axis, int m
     using F = typename P::template F<true>;
     const int grid = cdiv(h.N[1], 2 * LT) * h.N[2];
     if (h.fuse_xeos && mode == KWB_MODE_STEP)
-      kwb_launch(k_line_fast<F, true, LT, P::MINB, true>, grid, LT * F::G, pline_smem<F>(LT), st, h, axis, mode, s);
+      kwb_launch(k_line_fast<F, true, LT, min_ctas<N>(LT), true>, grid, LT * F::G, pline_smem<F>(LT), st, h, axis, mode, s);
     else
-      kwb_launch(k_line_fast<F, true, LT, P::MINB, false>, grid, LT * F::G, pline_smem<F>(LT), st, h, axis, mode, s);
+      kwb_launch(k_line_fast<F, true, LT, min_ctas<N>(LT), false>, grid, LT * F::G, pline_smem<F>(LT), st, h, axis, mode, s);
   } else {
     using F = typename P::template F<false>;
     const int grid = cdiv(h.N[0], 2 * LT) * (axis == 1 ? h.N[2] : h.N[1]);
@@ -2030,11 +2072,11 @@ static inline void line_go(const SimDev *d_sim, const SimDev &h, int axis, int m
       SimDev hs = h;
       if (encode_strided_maps(hs, axis, 2 * LT)) {
         hs.tile_tma_s = 1;
-        kwb_launch(k_line_fast<F, false, LT, P::MINB, false, true>, grid, LT * F::G, pline_smem<F>(LT), st, hs, axis, mode, s);
+        kwb_launch(k_line_fast<F, false, LT, min_ctas<N>(LT), false, true>, grid, LT * F::G, pline_smem<F>(LT), st, hs, axis, mode, s);
         return;
       }
     }
-    kwb_launch(k_line_fast<F, false, LT, P::MINB, false>, grid, LT * F::G, pline_smem<F>(LT), st, h, axis, mode, s);
+    kwb_launch(k_line_fast<F, false, LT, min_ctas<N>(LT), false>, grid, LT * F::G, pline_smem<F>(LT), st, h, axis, mode, s);
   }
 }
 
@@ -2066,11 +2108,11 @@ static inline cudaError_t prime_eos_variant() {
   using FC = typename P::template F<true>;
   using FS = typename P::template F<false>;
   cudaError_t e;
-  if ((e = raise_smem((const void *)k_eos_fwd_fast<FC, LT, P::MINB, false>, eos_smem<FC>(LT))) != cudaSuccess) return e;
-  if ((e = raise_smem((const void *)k_eos_inv_fast<FC, LT, P::MINB, false>, eos_smem<FC>(LT))) != cudaSuccess) return e;
-  if ((e = raise_smem((const void *)k_eos_fwd_fast<FC, LT, P::MINB, true>, eos_smem<FC>(LT))) != cudaSuccess) return e;
-  if ((e = raise_smem((const void *)k_eos_inv_fast<FC, LT, P::MINB, true>, eos_smem<FC>(LT))) != cudaSuccess) return e;
-  return raise_smem((const void *)k_spec_fast<FS, LT, P::MINB>, eos_smem<FS>(LT));
+  if ((e = raise_smem((const void *)k_eos_fwd_fast<FC, LT, min_ctas<N>(LT), false>, eos_smem<FC>(LT))) != cudaSuccess) return e;
+  if ((e = raise_smem((const void *)k_eos_inv_fast<FC, LT, min_ctas<N>(LT), false>, eos_smem<FC>(LT))) != cudaSuccess) return e;
+  if ((e = raise_smem((const void *)k_eos_fwd_fast<FC, LT, min_ctas<N>(LT), true>, eos_smem<FC>(LT))) != cudaSuccess) return e;
+  if ((e = raise_smem((const void *)k_eos_inv_fast<FC, LT, min_ctas<N>(LT), true>, eos_smem<FC>(LT))) != cudaSuccess) return e;
+  return raise_smem((const void *)k_spec_fast<FS, LT, min_ctas<N>(LT)>, eos_smem<FS>(LT));
 }
 
 template <int N>
@@ -2090,11 +2132,11 @@ static inline void eos_go(const SimDev *d_sim, const SimDev &h, bool fwd, long l
   using F = typename P::template F<true>;
   const int grid = cdiv(h.N[1], 2 * LT) * h.N[2];
   if (h.plane) {
-    if (fwd) kwb_launch(k_eos_fwd_fast<F, LT, P::MINB, true>, grid, LT * F::G, eos_smem<F>(LT), st, h, s);
-    else kwb_launch(k_eos_inv_fast<F, LT, P::MINB, true>, grid, LT * F::G, eos_smem<F>(LT), st, h, s);
+    if (fwd) kwb_launch(k_eos_fwd_fast<F, LT, min_ctas<N>(LT), true>, grid, LT * F::G, eos_smem<F>(LT), st, h, s);
+    else kwb_launch(k_eos_inv_fast<F, LT, min_ctas<N>(LT), true>, grid, LT * F::G, eos_smem<F>(LT), st, h, s);
   } else {
-    if (fwd) kwb_launch(k_eos_fwd_fast<F, LT, P::MINB, false>, grid, LT * F::G, eos_smem<F>(LT), st, h, s);
-    else kwb_launch(k_eos_inv_fast<F, LT, P::MINB, false>, grid, LT * F::G, eos_smem<F>(LT), st, h, s);
+    if (fwd) kwb_launch(k_eos_fwd_fast<F, LT, min_ctas<N>(LT), false>, grid, LT * F::G, eos_smem<F>(LT), st, h, s);
+    else kwb_launch(k_eos_inv_fast<F, LT, min_ctas<N>(LT), false>, grid, LT * F::G, eos_smem<F>(LT), st, h, s);
   }
 }
 
@@ -2117,7 +2159,7 @@ static inline void spec_go(const SimDev *d_sim, const SimDev &h, int axis, int o
   using P = LinePolicy<N>;
   using F = typename P::template F<false>;
   const int grid = cdiv(h.n1, LT) * (axis == 1 ? h.N[2] : h.N[1]);
-  kwb_launch(k_spec_fast<F, LT, P::MINB>, grid, LT * F::G, eos_smem<F>(LT), st, h, axis, op, s);
+  kwb_launch(k_spec_fast<F, LT, min_ctas<N>(LT)>, grid, LT * F::G, eos_smem<F>(LT), st, h, axis, op, s);
 }
 
 template <int N>
@@ -2381,11 +2423,11 @@ static inline void el_go(const SimDev &h, int axis, const ElGrad &g, long long s
   using P = LinePolicy<N>;
   if (axis == 0) {
     using F = typename P::template F<true>;
-    kwb_launch(k_el_grad_fast<F, true, LT, P::MINB>, cdiv(h.N[1], 2 * LT) * h.N[2], LT * F::G, pline_smem<F>(LT),
+    kwb_launch(k_el_grad_fast<F, true, LT, min_ctas<N>(LT)>, cdiv(h.N[1], 2 * LT) * h.N[2], LT * F::G, pline_smem<F>(LT),
                st, h, axis, g, s);
   } else {
     using F = typename P::template F<false>;
-    kwb_launch(k_el_grad_fast<F, false, LT, P::MINB>, cdiv(h.N[0], 2 * LT) * (axis == 1 ? h.N[2] : h.N[1]),
+    kwb_launch(k_el_grad_fast<F, false, LT, min_ctas<N>(LT)>, cdiv(h.N[0], 2 * LT) * (axis == 1 ? h.N[2] : h.N[1]),
                LT * F::G, pline_smem<F>(LT), st, h, axis, g, s);
   }
 }

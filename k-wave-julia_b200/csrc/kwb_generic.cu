@@ -12,8 +12,9 @@
 // stage functions), used for every stage of every transform, and everything that touches global
 // memory is a rolled loop over elements, four in flight a thread.  Stages fused with the field
 // updates (one unrolled body a radix and update) waited on instructions for 9 of 16 issue slots at
-// 120 x 108 x 100 and took 154 us a step; the Stockham stages of radix 2, 3, 4, 5, 7 and 8 before
-// them, one sweep and barrier a prime factor, 206 us.
+// 120 x 108 x 100 and took 154 us a step; Stockham stages of radix 2, 3, 4, 5, 7 and 8, one sweep and
+// barrier a prime factor, 206 us; these take 113 us (810 x 450: 102 -> 69 us), three CTAs of up to 256
+// threads an SM.
 #include <algorithm>
 
 #include "kwb_fft.cuh"
@@ -638,8 +639,8 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
 // and even, so that the inverse transform of the full spectrum is real as it stands -- with the
 // field updates between them.  Launched pass by pass, a step of 512 points cost four kernels of about
 // 5 us each (launch, first loads, tables), 20 us; what bounds it here is the chain of stages and
-// block barriers (about 20) of the three convolutions.  The steps of a launch keep p, u and rho in
-// shared memory; the medium and the operator tables stay in L1.
+// block barriers (about 20) of the three convolutions, 9.4 us.  The steps of a launch keep p, u and
+// rho in shared memory; the medium and the operator tables stay in L1.
 __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     k_steps_1d(const __grid_constant__ SimDev S, const __grid_constant__ Groups1D groups, long long t_first, int steps) {
   const FftPlan &pl = S.plan[0];

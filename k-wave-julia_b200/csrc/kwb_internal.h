@@ -192,12 +192,12 @@ struct SimDev {
   int num_sms;        // multiprocessors of the device (tile sizing)
   int tile_override;  // register-FFT tile variant forced for every pass (-1: chosen per pass)
   // Measured FFT schedule (kwb_tune.cu): register-FFT tile variant per pass slot (KWB_SLOT_*;
-  // -1: the size heuristic) and Stockham line-pass threads per CTA per axis (0: heuristic).
-  // Lines per tile (L_*) and the Stockham radix order (plan) are the other tuned choices.
+  // -1: the size heuristic) and in-place line-pass threads per CTA per axis (0: heuristic).
+  // Lines per tile (L_*) and the radix order (plan) are the other tuned choices.
   signed char tile_var[8];
   short thr_line[3];
-  signed char plan_order[3];  // make_plan_order's order of each axis's Stockham plan
-  int grid_fill;      // Stockham passes of small grids: narrower tiles and larger CTAs to fill the GPU
+  signed char plan_order[3];  // make_plan_order's order of each axis's plan
+  int grid_fill;      // in-place passes of small grids: narrower tiles to fill the GPU
 
   // Elastic solver (pstd_elastic_2d/3d).  u[d] are the velocities, p the recorded pressure
   // -trace(sigma)/D.  el_s: stresses in the slots xx, yy, zz, xy, xz, yz (2-D: 0, 1, 3).  el_w:
@@ -472,7 +472,7 @@ bool schedule_parse(const char *txt, Schedule &s);
 // Measure every pass of h's time step under its candidate schedules (pick >= 0: take candidate
 // `pick` of every pass instead) and store the fastest in h.  Runs on h's own field and spectrum
 // buffers, which the caller must reset afterwards; d_scratch holds the timing descriptor.
-// explore_order adds the Stockham radix orders (not bit-identical to the default order).
+// explore_order adds the radix orders (not bit-identical to the default order).
 cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pick, bool explore_order,
                           std::string *log);
 

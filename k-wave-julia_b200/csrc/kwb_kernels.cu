@@ -4,6 +4,9 @@
 // 296-535) is executed as:
 //
 //   [k_tr_inject]                      time-reversal injection (first_order.jl:450-460, 678-689)
+// (k_line_pass, k_eos_x_*, k_spec_pass: kwb_generic.cu, or for the lengths of kwb_fast.cu its register
+// passes; this file holds the others and the launchers that choose)
+//
 //   k_line_pass(axis) for every axis   fused: d/dx_d p -> u_d update (split PML) -> u source ->
 //                                      d/dx_d u_d -> rho_d update (split PML) -> p source
 //                                      (first_order_steps.jl:400-428, 489-521, 586-715)

@@ -13,8 +13,8 @@
 //     loads libkwb holds it until the process exits, used or not;
 //   * the half spectrum must fit: (Nx/2 + 1) * Ny * Nz <= KWB_NOALLOC_MAX_SPECTRUM (2,621,440,
 //     e.g. 2048 x 2048, or 160^3); larger grids are rejected with KWB_E_UNSUPPORTED;
-//   * the dispersion branch (scalar c0 with :stokes absorption) needs a second spectrum and the
-//     previous density and is not offered here;
+//   * the dispersion branch (scalar c0 with :stokes absorption) needs the spectrum of the
+//     step before and is not offered here;
 //   * every call shares the array, so calls whose GPU work overlaps (different streams, threads
 //     or processes sharing a device context) race on it and must be serialised by the caller.
 #include <cmath>

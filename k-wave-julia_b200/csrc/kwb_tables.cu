@@ -1,10 +1,10 @@
 // FP64 operator-table builders.  Every table is computed in double precision on the device and
 // rounded once to FP32:
-//   * twiddles exp(-2 pi i m/N)                             (the FFT engine, kwb_fft.cuh)
+//   * twiddles exp(-2 pi i m/N)                             (the FFT kernels)
 //   * gradient multipliers i k e^{+-i k d/2} / N           (fft_utils.jl:247-303, grid.jl:120-153)
 //   * PML deficits 1 - exp(-alpha pos^4 dt)                (pml.jl:25-56)
 //   * EOS multiplier [c^2] kappa (1 + tau |k|^y) / Ntot and
-//     the dispersion multiplier c^2 kappa eta |k|^(y-1) / Ntot   (solver/first_order.jl:13-42,
+//     with dispersion the two multipliers that it takes       (solver/first_order.jl:13-42,
 //                                                             solver/first_order_steps.jl:243-286)
 //   * medium conversions (c0^2, Q = BonA/(2 rho0)) and source signal tables p/(D c^2).
 #include "kwb_internal.h"

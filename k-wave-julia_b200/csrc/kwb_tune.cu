@@ -7,12 +7,13 @@
 //     tiles --, for the line passes whether the tiles are staged by TMA copies or by 16-byte
 //     cp.async, and, for the 3-D cluster plane pass, 8 CTAs of 512 threads or 16 of 256 per plane
 //     with row-major or slot-major rows;
-//   * Stockham passes (other lengths): the radix order of each axis's plan, the complex lines per
-//     tile, and the threads per CTA of the line passes.
+//   * in-place passes (other lengths): the radix order of each axis's plan, the complex lines per
+//     tile, and the threads per CTA of the line passes;
+//   * the elastic solver's gradient passes: the tile variant of each axis.
 // Each candidate runs on the simulation's own buffers before its initial conditions are set
 // (sensors, sources and time reversal are switched off in the timing descriptor): one warm-up
-// time step, then three timed with CUDA events, so that a candidate is judged by the step it
-// gives; the passes are tuned one at a time, each with the others at their current choice.  Every candidate computes the same transform: the tile shape
+// time step, then three timed with CUDA events (on grids of up to 4 Mi points a replayed graph of
+// 16 steps, as the simulation runs them), so that a candidate is judged by the step it gives; the passes are tuned one at a time, each with the others at their current choice.  Every candidate computes the same transform: the tile shape
 // and thread count leave the arithmetic of each line unchanged, so results are bit-identical
 // whatever is picked -- a simulation gives the same fields alone, tuned, and in a batch, which
 // keeps the heuristic.  A different radix order only reorders FP32 rounding; it is explored
@@ -110,23 +111,43 @@ struct Tuner {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   std::string *log;
 
-  // Average device time of one launch of `go` with the descriptor t (FLT_MAX if it failed).
+  // Average device time of one launch of `go` (a time step) with the descriptor t (FLT_MAX if it
+  // failed).  Grids whose steps take tens of microseconds are timed as their simulation runs them,
+  // from a replayed graph: launched one by one, a 512^2 step took the host's 20 us whatever its
+  // tiles, and the choice was left to noise (128^2: 15.0 or 18.2 us a step).
   template <class F>
   float time(F go) {
     cudaError_t e = cudaMemcpyAsync(d_t, &t, sizeof(SimDev), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = t.elastic ? el_prime(t) : prime_attributes(t);
     if (e == cudaSuccess) e = go();
+    const int reps = t.nvox <= (4LL << 20) ? 16 : 3;
+    cudaGraphExec_t ex = nullptr;
+    if (reps > 3 && e == cudaSuccess) {
+      cudaGraph_t g = nullptr;
+      e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+      for (int r = 0; r < reps && e == cudaSuccess; ++r) e = go();
+      const cudaError_t e2 = cudaStreamEndCapture(st, &g);
+      if (e == cudaSuccess) e = e2;
+      if (e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
+      if (g) cudaGraphDestroy(g);
+      if (e == cudaSuccess) e = cudaGraphLaunch(ex, st);
+    }
     if (e == cudaSuccess) e = cudaEventRecord(e0, st);
-    for (int r = 0; r < 3 && e == cudaSuccess; ++r) e = go();
+    if (ex && e == cudaSuccess) e = cudaGraphLaunch(ex, st);
+    for (int r = 0; !ex && r < reps && e == cudaSuccess; ++r) e = go();
     if (e == cudaSuccess) e = cudaEventRecord(e1, st);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+    if (ex) {
+      cudaStreamSynchronize(st);
+      cudaGraphExecDestroy(ex);
+    }
     float ms = 0.f;
     if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return FLT_MAX;
     }
-    return ms / 3.f;
+    return ms / (float)reps;
   }
 
   // Try `n` candidates set by set(i) (i < n), keep the fastest (or candidate `pick`).
@@ -237,7 +258,7 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
         T.choose("line_tma", 2, [&, a](int i) { t.tma_line[a] = (signed char)(i == 0 ? 0 : 1); }, go);
       continue;
     }
-    // Stockham: radix order (distinct plans only; with explore_order), then lines per tile,
+    // in-place passes: radix order (distinct plans only; with explore_order), then lines per tile,
     // then threads per CTA
     std::vector<int> orders;
     std::vector<FftPlan> plans;
@@ -259,6 +280,17 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
     T.choose("line_L", (int)Ls.size(), [&, a](int i) { t.L_line[a] = Ls[i]; }, go);
     const int thr[4] = {0, 64, 128, 256};
     T.choose("line_threads", 4, [&, a](int i) { t.thr_line[a] = (short)thr[i]; }, go);
+  }
+
+  // y and z together: their passes are alike and run one after the other, and two that change together
+  // can be faster where either alone is not (160^3: 128-thread tiles on both 217 us a step, on one or
+  // neither 241-249)
+  if (D == 3 && line_is_fast(t, 1) && line_is_fast(t, 2)) {
+    const signed char y = t.tile_var[KWB_SLOT_LINE1], z = t.tile_var[KWB_SLOT_LINE2];
+    T.choose("line_yz_tile", 4, [&](int i) {
+      t.tile_var[KWB_SLOT_LINE1] = i == 0 ? y : (signed char)(i - 1);
+      t.tile_var[KWB_SLOT_LINE2] = i == 0 ? z : (signed char)(i - 1);
+    }, step);
   }
 
   // equation of state, x direction
