@@ -34,6 +34,11 @@ struct kwb_ctx {
   // pinned staging for device -> host read-back (two halves), allocated on first use
   float *pin = nullptr;
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
+  // ... or, while only pressure fields have been read back, halves of their size (pinning the full
+  // buffer takes 28 ms)
+  float *pin_field = nullptr;
+  long long pin_field_half = 0;  // floats
+  std::mutex pin_mu;             // pressure fields of several simulations may be read from several threads
   // Device memory pool of this context's simulations: stream-ordered allocation, and freed
   // blocks stay in the pool for the next simulation (no unmapping between simulations).
   cudaMemPool_t pool = nullptr;
@@ -43,6 +48,7 @@ struct kwb_ctx {
   ~kwb_ctx() {
     if (pool) cudaMemPoolDestroy(pool);  // released once outstanding blocks are freed
     if (pin) cudaFreeHost(pin);
+    if (pin_field) cudaFreeHost(pin_field);
     for (cudaEvent_t e : pin_ev)
       if (e) cudaEventDestroy(e);
   }
@@ -103,14 +109,30 @@ constexpr long long kPinFloats = 8LL << 20;  // floats per half of the pinned bu
 template <class Sink>
 int read_chunks(kwb_ctx *ctx, cudaStream_t st, const float *src, long long cnt, long long chunk, Sink &&sink) {
   if (cnt <= 0) return KWB_OK;
-  if (!ctx->pin) {
+  std::lock_guard<std::mutex> lk(ctx->pin_mu);
+  for (cudaEvent_t &e : ctx->pin_ev)
+    if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  float *buf = ctx->pin;
+  long long half = kPinFloats;
+  if (!buf && chunk < kPinFloats) {
+    half = std::min(chunk, cnt);
+    if (ctx->pin_field_half < half) {
+      if (ctx->pin_field) cudaFreeHost(ctx->pin_field);
+      ctx->pin_field = nullptr;
+      ctx->pin_field_half = 0;
+      CU(cudaMallocHost(&ctx->pin_field, 2 * half * sizeof(float)));
+      ctx->pin_field_half = half;
+    }
+    buf = ctx->pin_field;
+    half = ctx->pin_field_half;
+  } else if (!buf) {
     CU(cudaMallocHost(&ctx->pin, 2 * kPinFloats * sizeof(float)));
-    for (cudaEvent_t &e : ctx->pin_ev) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    buf = ctx->pin;
   }
   const long long nch = (cnt + chunk - 1) / chunk;
   auto issue = [&](long long c) -> cudaError_t {
     const long long lo = c * chunk, len = std::min(chunk, cnt - lo);
-    cudaError_t e = cudaMemcpyAsync(ctx->pin + (c & 1) * kPinFloats, src + lo, len * 4, cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaMemcpyAsync(buf + (c & 1) * half, src + lo, len * 4, cudaMemcpyDeviceToHost, st);
     return e == cudaSuccess ? cudaEventRecord(ctx->pin_ev[c & 1], st) : e;
   };
   CU(issue(0));
@@ -118,7 +140,7 @@ int read_chunks(kwb_ctx *ctx, cudaStream_t st, const float *src, long long cnt, 
     CU(cudaEventSynchronize(ctx->pin_ev[c & 1]));
     if (c + 1 < nch) CU(issue(c + 1));
     const long long lo = c * chunk;
-    sink(ctx->pin + (c & 1) * kPinFloats, lo, std::min(chunk, cnt - lo));
+    sink(buf + (c & 1) * half, lo, std::min(chunk, cnt - lo));
   }
   return KWB_OK;
 }
@@ -655,10 +677,10 @@ int upload(kwb_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t 
     CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
     return KWB_OK;
   }
-  if (!ctx->pin) {
-    CU(cudaMallocHost(&ctx->pin, 2 * half));
-    for (cudaEvent_t &e : ctx->pin_ev) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  }
+  std::lock_guard<std::mutex> lk(ctx->pin_mu);
+  if (!ctx->pin) CU(cudaMallocHost(&ctx->pin, 2 * half));
+  for (cudaEvent_t &e : ctx->pin_ev)
+    if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   const size_t nch = (bytes + half - 1) / half;
   for (size_t c = 0; c < nch; ++c) {
     char *pin = reinterpret_cast<char *>(ctx->pin) + (c & 1) * half;
