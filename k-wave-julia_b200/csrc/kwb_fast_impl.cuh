@@ -317,7 +317,9 @@ struct LineFFT3G {
   __host__ __device__ static constexpr int nat(int k) { return k + (k >> 5); }
   static constexpr int S1 = (R1 - 1) * RP1 + G, S2 = (R1 - 1) * Q2 + (B - 1) * M2 + A, S3 = N + (N >> 5);
   static constexpr int SM = S1 > S2 ? (S1 > S3 ? S1 : S3) : (S2 > S3 ? S2 : S3);
-  static constexpr int LP = SM | 1;
+  // odd, so that the lines of a strided warp differ; lines of 8 threads held by one warp take
+  // consecutive slots, two of which fill the banks when 8 apart
+  static constexpr int LP = WARP && G == 8 ? (SM + 7) / 16 * 16 + 8 : SM | 1;
   static constexpr int TW = R1 * RP + B * AP;
   __device__ __forceinline__ static int i1(int q, int u) { return q * RP1 + u; }
   __device__ __forceinline__ static int i2(int q1, int mb, int a) { return q1 * Q2 + mb * M2 + a; }
@@ -630,6 +632,13 @@ __global__ void __launch_bounds__(256)
     pm[F::N + i] = pml[i];
   }
 }
+// Row pitch of a staged contiguous tile: where a warp reads several lines (G < 32 threads each), the
+// two rows a line apart must not fall in the same banks (160 points, four lines a warp: 7.5 of 12.3
+// million shared-memory wavefronts of the x pass were conflicts).
+template <class F>
+__host__ __device__ constexpr int row_pitch() {
+  return F::N + (F::G >= 32 ? 0 : F::G >= 8 ? (F::G / 2) & ~3 : 4);
+}
 // Register line pass: exchange buffers and table image, then the two staged operand tiles,
 // 128-byte aligned (destinations of tiled TMA copies).
 template <class F>
@@ -638,7 +647,7 @@ __host__ __device__ constexpr size_t pline_offset(int L) {
 }
 template <class F>
 __host__ __device__ constexpr size_t pline_smem(int L) {
-  return pline_offset<F>(L) + 2 * (size_t)(2 * L) * F::N * sizeof(float);
+  return pline_offset<F>(L) + 2 * (size_t)(2 * L) * row_pitch<F>() * sizeof(float);
 }
 
 // 16-byte asynchronous global->shared copy; bytes beyond src_bytes are zero-filled.
@@ -817,18 +826,23 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   // table set-up and, for rho0, the first transform.  Staged layout: CONTIG [row][i],
   // strided [i][column] (the tile's own global layout, compacted).
   float *st_p = reinterpret_cast<float *>(reinterpret_cast<char *>(smem_raw) + pline_offset<F>(L));
-  float *st_r = st_p + 2 * L * N;
+  constexpr int NP = CONTIG ? row_pitch<F>() : N;
+  float *st_r = st_p + 2 * L * NP;
   // Chunk assignments are compile-time strides from a per-thread start, so the addresses of a
   // thread's chunks differ by constants.
   auto stage = [&](float *dst, const float *f, int slot) {
     const float *fb = f + base;
     if (CONTIG && tma) {
-      // rows contiguous in memory: one bulk copy of cnt rows (16-byte aligned: N % 4 == 0)
+      // rows contiguous in memory: one bulk copy each, or all in one (16-byte aligned: N % 4 == 0)
       if (tid == 0) {
         const unsigned bytes = (unsigned)cnt * N * 4u;
         fence_proxy_async_smem();
         mbar_expect_tx(&tile_bar[slot], bytes);
-        if (!(S.test_drop_copy && slot == 0 && blockIdx.x == 0)) bulk_copy_g2s(dst, fb, bytes, &tile_bar[slot]);
+        if (!(S.test_drop_copy && slot == 0 && blockIdx.x == 0)) {
+          if constexpr (NP == N) bulk_copy_g2s(dst, fb, bytes, &tile_bar[slot]);
+          else
+            for (int r = 0; r < cnt; ++r) bulk_copy_g2s(dst + r * NP, fb + r * N, N * 4u, &tile_bar[slot]);
+        }
       }
       return;
     } else if (!CONTIG && tma) {
@@ -856,7 +870,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
         const int q = tid + k * THREADS;
-        if (q < chunks) cp_async16(dst + 4 * q, fb + 4 * q, 16);
+        if (q < chunks) cp_async16(dst + 4 * q + (q / (N / 4)) * (NP - N), fb + 4 * q, 16);
       }
     } else {
       constexpr int CPR = (2 * L) / 4;  // 16-byte chunks per tile row (strided tiles have L >= 2)
@@ -897,7 +911,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     return ok;
   };
   auto staged = [&](const float *st, int i) -> float2 {
-    if (CONTIG) return make_float2(va ? st[(2 * l) * N + i] : 0.f, vb ? st[(2 * l + 1) * N + i] : 0.f);
+    if (CONTIG) return make_float2(va ? st[(2 * l) * NP + i] : 0.f, vb ? st[(2 * l + 1) * NP + i] : 0.f);
     return *reinterpret_cast<const float2 *>(st + i * 2 * L + 2 * l);
   };
   const float *__restrict__ rho0 = S.rho0;
@@ -906,7 +920,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   // memory (entry by entry at the point of use, a chain of three loads each, they held the tiles of
   // a 9 x 9 disc source up by 3-4 us a pass).  More than SRC_CAP entries on a tile are read in
   // place.
-  constexpr int SRC_CAP = 128, SRC_PER = (SRC_CAP + THREADS - 1) / THREADS;
+  constexpr int SRC_CAP = 96, SRC_PER = (SRC_CAP + THREADS - 1) / THREADS;
   __shared__ int src_ptr[2][2 * LT + 1];
   __shared__ int2 src_ent[2][SRC_CAP];  // line << 16 | position, value
   const bool has_u = mode == KWB_MODE_STEP && S.u_sig[axis] && S.u_line_ptr[axis];
@@ -1335,12 +1349,11 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     qb = __ldg(lp + 1);
     qc = vb ? __ldg(lp + 2) : qb;
   }
-  int2 ent_a = make_int2(0, 0), ent_b = ent_a;  // this thread's first point on either row
-  if (tt < qb - qa) ent_a = __ldg(gs->line_ent + qa + tt);
-  if (tt < qc - qb) ent_b = __ldg(gs->line_ent + qb + tt);
-  const unsigned gs_mask = gs ? gs->mask : 0u;
-  const long long gs_n = gs ? gs->n : 0;
-  float *const gs_ser = gs ? gs->ser_p : nullptr;
+  // this thread's first point on either row (not beside the plane pass: a 256^3 pass has other warps
+  // to run, and the registers cost it 51.6 -> 56.7 us)
+  int2 ent_a = make_int2(0, 0), ent_b = ent_a;
+  if (!PLANE && tt < qb - qa) ent_a = __ldg(gs->line_ent + qa + tt);
+  if (!PLANE && tt < qc - qb) ent_b = __ldg(gs->line_ent + qb + tt);
   pdl_wait();
   const long long t = *S.t0 + step_s;
   // The half spectrum's rows, all of a thread's loads in flight at once (k = tt + G j, and the
@@ -1480,17 +1493,17 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
 #pragma unroll
     for (int r = 0; r < E; ++r) xs[tt + G * r] = v[r];
     F::sync();
-    const unsigned sm_ = gs_mask;
+    const unsigned sm_ = gs->mask;
     const bool last = (t == S.Nt - 1);
     for (int c = 0; c < 2; ++c) {
       if (!(c ? vb : va)) continue;
       const int q0 = c ? qb : qa, q1 = c ? qc : qb;
       for (int q = q0 + tt; q < q1; q += G) {
-        const int2 e = q - q0 >= G ? gs->line_ent[q] : c ? ent_b : ent_a;
+        const int2 e = PLANE || q - q0 >= G ? gs->line_ent[q] : c ? ent_b : ent_a;
         const float2 pp = xs[e.x];
         const float pv = c ? pp.y : pp.x;
         const long long j = e.y;
-        if (sm_ & (1u << 0)) gs_ser[t * gs_n + j] = pv;
+        if (sm_ & (1u << 0)) gs->ser_p[t * gs->n + j] = pv;
         if (sm_ & (1u << 1)) gs->pmax[j] = fmaxf(gs->pmax[j], pv);
         if (sm_ & (1u << 2)) gs->pmin[j] = fminf(gs->pmin[j], pv);
         if (sm_ & (1u << 3)) gs->prms[j] += (double)gs->cnt_prms * ((double)pv * (double)pv);
@@ -2335,7 +2348,8 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   const bool va = 2 * l < cnt, vb = 2 * l + 1 < cnt;
   auto off = [&](int c, int i) -> int { return CONTIG ? c * Nx + i : i * st32 + c; };
   float *st0 = reinterpret_cast<float *>(reinterpret_cast<char *>(smem_raw) + pline_offset<F>(L));
-  float *st1 = st0 + 2 * L * N;
+  constexpr int NP = CONTIG ? row_pitch<F>() : N;
+  float *st1 = st0 + 2 * L * NP;
   auto stage = [&](float *dst, const float *f) {
     const float *fb = f + base;
     if (CONTIG) {
@@ -2344,7 +2358,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
 #pragma unroll
       for (int k = 0; k < PER; ++k) {
         const int q = tid + k * THREADS;
-        if (q < chunks) cp_async16(dst + 4 * q, fb + 4 * q, 16);
+        if (q < chunks) cp_async16(dst + 4 * q + (q / (N / 4)) * (NP - N), fb + 4 * q, 16);
       }
     } else {
       constexpr int CPR = (2 * L) / 4;
@@ -2363,7 +2377,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   };
 
   auto staged = [&](const float *st, int i) -> float2 {
-    if (CONTIG) return make_float2(va ? st[(2 * l) * N + i] : 0.f, vb ? st[(2 * l + 1) * N + i] : 0.f);
+    if (CONTIG) return make_float2(va ? st[(2 * l) * NP + i] : 0.f, vb ? st[(2 * l + 1) * NP + i] : 0.f);
     return *reinterpret_cast<const float2 *>(st + i * 2 * L + 2 * l);
   };
   // the destination as this kernel may already have written it: ordinary (coherent) loads

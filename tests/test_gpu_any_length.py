@@ -63,8 +63,8 @@ def test_dispersion_from_the_last_spectrum(shape, nonlinear):
     check(make_case(shape, seed=7, stokes=True, nonlinear=nonlinear))
 
 
-# the register passes hold up to 128 source entries of a tile in shared memory and read more in place
-@pytest.mark.parametrize("points", [1, 40, 127, 129, 2000])
+# the register passes hold up to 96 source entries of a tile in shared memory and read more in place
+@pytest.mark.parametrize("points", [1, 40, 95, 127, 129, 2000])
 @pytest.mark.parametrize("source", ["p", "u"])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_source_entries_of_a_tile(points, source, mode):
