@@ -363,15 +363,16 @@ std::vector<float2> gradient_conv(const FftPlan &pl, double d, int sign) {
   const double pi = 3.141592653589793238462643;
   const int n = pl.n, m = pl.m;
   std::vector<double> h(n, 0.0);
-  std::vector<cplx> w(2 * n);  // exp(i pi j/n)
-  for (int j = 0; j < 2 * n; ++j) w[j] = cplx(std::cos(pi * j / n), std::sin(pi * j / n));
-  for (int k = 0; k < n; ++k) {
-    const int ks = k < (n + 1) / 2 ? k : k - n;
-    const double kv = 2.0 * pi * ks / (n * d);
-    // k (2 j +- 1) pi / n
+  std::vector<double> sn(2 * n);  // sin(pi j/n)
+  for (int j = 0; j < 2 * n; ++j) sn[j] = std::sin(pi * j / n);
+  // k and -k give the same term, the Nyquist bin of an even length one
+  for (int k = 1; k <= n / 2; ++k) {
+    const double kv = (2 * k == n ? 1.0 : 2.0) * 2.0 * pi * k / (n * d);
+    int q = sign > 0 ? k : 2 * n - k;  // k (2 j +- 1) mod 2n
     for (int j = 0; j < n; ++j) {
-      const long long q = ((long long)ks * (2 * j + sign)) % (2 * n);
-      h[j] -= kv * w[q < 0 ? q + 2 * n : q].imag();
+      h[j] -= kv * sn[q];
+      q += 2 * k;
+      if (q >= 2 * n) q -= 2 * n;
     }
   }
   std::vector<cplx> hk(m, 0.0);
