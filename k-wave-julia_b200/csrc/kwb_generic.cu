@@ -10,10 +10,10 @@
 // What bounds these passes is instruction fetch: a radix body is some 300 unrolled instructions,
 // run by few warps.  So there is one copy of each body for all kernels of this file (the noinline
 // stage functions), used for every stage of every transform, and everything that touches global
-// memory is a rolled loop over elements, four in flight a thread.  Stages fused with the field
+// memory is a rolled loop over elements, two in flight a thread.  Stages fused with the field
 // updates (one unrolled body a radix and update) waited on instructions for 9 of 16 issue slots at
 // 120 x 108 x 100 and took 154 us a step; Stockham stages of radix 2, 3, 4, 5, 7 and 8, one sweep and
-// barrier a prime factor, 206 us; these take 113 us (810 x 450: 102 -> 69 us), three CTAs of up to 256
+// barrier a prime factor, 206 us; these take 112 us (810 x 450: 102 -> 66 us), three CTAs of up to 256
 // threads an SM.
 #include <algorithm>
 
@@ -176,8 +176,9 @@ __device__ __forceinline__ PassSmem pass_smem(const FftPlan &pl, const float2 *t
 
 // Elements of the tile, UNROLL a thread at a time: load(j, l, i) for each, then use(j, l, i). Element
 // i of line l; neighbouring lanes take neighbouring positions (BYROW) or lines.  A thread's last
-// round may repeat its first element's load.
-constexpr int UNROLL = 4;
+// round may repeat its first element's load.  (810 x 450 / 120 x 108 x 100, us a step: unrolled once
+// 69.6 / 116.8, twice 66.3 / 112, three times 67.0 / 113.2, four times 68.7 / 113.6, eight 83.7 / 128.)
+constexpr int UNROLL = 2;
 template <bool BYROW, class Load, class Use>
 __device__ __forceinline__ void elements(int L, int n, FastDiv dL, FastDiv dn, Load &&load, Use &&use) {
   const int total = L * n;
