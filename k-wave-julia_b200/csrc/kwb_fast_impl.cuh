@@ -659,7 +659,8 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Copy `bytes` (a multiple of 16) of an axis's table image into shared memory, as one group.  The
+// Copy `bytes` (a multiple of 16) of an axis's table image into shared memory (16-byte aligned, so an
+// even number of pairs after its start: every tile has an even number of lines), as one group.  The
 // copies allocate in L1 (.ca): the CTAs that follow on an SM take the image from there.
 __device__ __forceinline__ void stage_image(void *dst, const float2 *img, size_t bytes) {
   for (unsigned c = threadIdx.x; c < (unsigned)(bytes / 16); c += blockDim.x)
@@ -1663,6 +1664,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   constexpr int NY = FY::N, NZ = FZ::N, RZ = NZ / CL, CY = NY / CL;
   constexpr int LY = THREADS / FY::G, LZ = THREADS / FZ::G;
   static_assert(RZ == 2 * LY && CY % LZ == 0 && NZ % RZ == 0, "plane tiling");
+  static_assert(FY::TW % 2 == 0 && FZ::TW % 2 == 0, "twiddles in 16-byte pieces");
   constexpr int XS = (LY * FY::LP > LZ * FZ::LP) ? LY * FY::LP : LZ * FZ::LP;
   extern __shared__ __align__(128) float4 smem_raw[];
   float2 *data = reinterpret_cast<float2 *>(smem_raw);  // [RZ][NY]
@@ -2110,9 +2112,10 @@ static inline cudaError_t launch_line_n(const SimDev *d_sim, const SimDev &h, in
   return cudaGetLastError();
 }
 
+// (the twiddles as stage_image copies them, in whole 16-byte pieces: 400 points have an odd number)
 template <class F>
 __host__ __device__ constexpr size_t eos_smem(int L) {
-  return ((size_t)L * F::LP + F::TW) * sizeof(float2);
+  return (size_t)L * F::LP * sizeof(float2) + image_tw_bytes<F>();
 }
 
 template <int N, int LT>
