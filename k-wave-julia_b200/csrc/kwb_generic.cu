@@ -39,7 +39,7 @@ struct Lines {
 template <class Op>
 __device__ __forceinline__ void radix_switch(int R, Op &&op) {
   switch (R) {
-    case 1: break;  // (lengths of one stage begin with a 1)
+    case 1: op(std::integral_constant<int, 1>{}); break;
     case 2: op(std::integral_constant<int, 2>{}); break;
     case 3: op(std::integral_constant<int, 3>{}); break;
     case 4: op(std::integral_constant<int, 4>{}); break;
@@ -89,7 +89,8 @@ __device__ __noinline__ void stage(Lines ln, int R_, int st, int ts, int nb, Fas
   });
 }
 
-// The last forward stage, the multiply by g (digit-reversed order) and the first backward stage.
+// The last forward stage, the multiply by g (digit-reversed order) and the first backward stage.  A line
+// of one point has radix 1 here too: its transforms are nothing, but g still multiplies it.
 __device__ __noinline__ void stage_top(Lines ln, int R_, int nb, const float2 *__restrict__ g) {
   radix_switch(R_, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
@@ -113,6 +114,7 @@ __device__ __noinline__ void stage_top(Lines ln, int R_, int nb, const float2 *_
 
 template <bool INV>
 __device__ __forceinline__ void run_stage(const Lines &ln, const FftPlan &pl, int s) {
+  if (pl.radix[s] == 1) return;  // (lengths of one stage begin with a 1)
   stage<INV>(ln, pl.radix[s], pl.stride[s], pl.tstride[s], ln.L * pl.nbf[s], pl.div_st[s]);
   __syncthreads();
 }
