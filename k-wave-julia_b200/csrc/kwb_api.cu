@@ -39,6 +39,7 @@ struct kwb_ctx {
   float *pin_field = nullptr;
   long long pin_field_half = 0;  // floats
   std::mutex pin_mu;             // pressure fields of several simulations may be read from several threads
+                                 // (held for the transfers only, never while a stream computes)
   // Device memory pool of this context's simulations: stream-ordered allocation, and freed
   // blocks stay in the pool for the next simulation (no unmapping between simulations).
   cudaMemPool_t pool = nullptr;
@@ -109,6 +110,9 @@ constexpr long long kPinFloats = 8LL << 20;  // floats per half of the pinned bu
 template <class Sink>
 int read_chunks(kwb_ctx *ctx, cudaStream_t st, const float *src, long long cnt, long long chunk, Sink &&sink) {
   if (cnt <= 0) return KWB_OK;
+  // what the stream still computes is waited for first: under the lock, and with a copy queued behind
+  // it, it would hold up every other read-back and upload of the context
+  CU(cudaStreamSynchronize(st));
   std::lock_guard<std::mutex> lk(ctx->pin_mu);
   for (cudaEvent_t &e : ctx->pin_ev)
     if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

@@ -1,8 +1,10 @@
-"""Edges of the accepted range: grids with one-point sides.
+"""Edges of the accepted range: grids with one-point sides; reads of one simulation while another runs.
 
 Tolerance as in test_gpu_any_length.py: about ten transforms a step, each adding some 2e-7 of relative
 rounding error, below 3e-5 over 60 steps.
 """
+import threading
+
 import numpy as np
 import pytest
 
@@ -38,3 +40,48 @@ def test_elastic_one_point_sides(shape):
                   pml_size=0)
 
     assert_parity(run(kb), run(K), TOL_L2, TOL_MAX)
+
+
+@pytest.mark.parametrize("other", ["read", "create"])
+def test_reading_a_busy_simulation_holds_up_no_other_thread(other):
+    """pressure() of a simulation with a long queue of steps (40000 at 512^2, half a second) waits for them;
+    a second thread that reads an idle simulation of the same context, or creates one whose fields go
+    through the pinned buffer (8 MiB), is done before the first has its field."""
+    import kwave_b200 as kb
+
+    def sim(n):
+        rng = np.random.default_rng(n)
+        g = kb.KWaveGrid(n, 1e-4, n, 1e-4)
+        g.dt, g.Nt = 2e-8, 10 ** 6
+        return kb.Simulation(g, kb.KWaveMedium(sound_speed=1500.0 + 10.0 * rng.random((n, n)), density=1000.0),
+                             kb.KWaveSource(p0=1e5 * rng.random((n, n))), kb.KWaveSensor())
+
+    busy, idle = sim(512), sim(512)
+    sim(1024).close()  # its schedule is measured now
+    for s in (busy, idle):
+        s.advance(64)
+        s.sync()
+    alone = idle.pressure()
+    order, field, queued = [], {}, threading.Event()
+
+    def long_read():
+        busy.advance(40000)
+        queued.set()
+        field["busy"] = busy.pressure()
+        order.append("busy")
+
+    th = threading.Thread(target=long_read)
+    th.start()
+    queued.wait()
+    if other == "read":
+        field["idle"] = idle.pressure()
+    else:
+        sim(1024).close()
+    order.append("other")
+    th.join()
+    assert order == ["other", "busy"]
+    if other == "read":
+        assert np.array_equal(field["idle"], alone)
+    assert np.array_equal(busy.pressure(), field["busy"]) and np.isfinite(field["busy"]).all()
+    busy.close()
+    idle.close()
