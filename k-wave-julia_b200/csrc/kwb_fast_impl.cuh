@@ -2032,7 +2032,7 @@ static inline cudaError_t prime_line_variant() {
   using P = LinePolicy<N>;
   using F = typename P::template F<C>;
   cudaError_t e = raise_smem((const void *)k_line_fast<F, C, LT, min_ctas<N>(LT), false>, pline_smem<F>(LT));
-  if (e == cudaSuccess) e = raise_smem((const void *)k_el_grad_fast<F, C, LT, min_ctas<N>(LT)>, pline_smem<F>(LT));
+  if (e == cudaSuccess) e = raise_smem((const void *)k_el_grad_fast<F, C, LT, P::MINB>, pline_smem<F>(LT));
   if constexpr (C) {
     if (e == cudaSuccess) e = raise_smem((const void *)k_line_fast<F, C, LT, min_ctas<N>(LT), true>, pline_smem<F>(LT));
   } else {
@@ -2306,6 +2306,10 @@ inline cudaError_t plane_launch(const SimDev &h, long long s, cudaStream_t st) {
 // The fields go through the two staging slots in turn: field f + 1 lands while field f is
 // transformed, and field f + 2 takes field f's slot once every thread holds field f.  Each
 // derivative is written, or added to the destination (bit f of g.acc).
+// CTAs an SM: the full-width tile's for every width (not min_ctas): a thread holds a running sum beside
+// its transform, which narrow tiles held to 64 or 128 registers cannot load ahead of time (narrow
+// tiles, us a step: 1024^2 66 against 81, 64 x 256 x 64 107 against 122, 128^3 in 128-thread tiles
+// 151 against 161; 512^2 24.0 against 23.9).
 template <class F, bool CONTIG, int LT, int MINB>
 __global__ void __launch_bounds__(LT * F::G, MINB)
     k_el_grad_fast(const __grid_constant__ SimDev S, int axis, const __grid_constant__ ElGrad g, long long step_s) {
@@ -2383,11 +2387,13 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
     if (CONTIG) return make_float2(va ? st[(2 * l) * NP + i] : 0.f, vb ? st[(2 * l + 1) * NP + i] : 0.f);
     return *reinterpret_cast<const float2 *>(st + i * 2 * L + 2 * l);
   };
-  // the destination as this kernel may already have written it: ordinary (coherent) loads
+  // the destination as this kernel may already have written it: ordinary (coherent) loads, all of them
+  // after the dependency wait.  (As __ldcg they stay behind the barriers around them and no longer run
+  // under the inverse transform.)
   auto load_cur = [&](const float *f, int i) -> float2 {
     const float *fb = f + base;
-    if (!CONTIG) return vb ? __ldcg(reinterpret_cast<const float2 *>(fb + off(2 * l, i))) : make_float2(0.f, 0.f);
-    return make_float2(va ? __ldcg(fb + off(2 * l, i)) : 0.f, vb ? __ldcg(fb + off(2 * l + 1, i)) : 0.f);
+    if (!CONTIG) return vb ? *reinterpret_cast<const float2 *>(fb + off(2 * l, i)) : make_float2(0.f, 0.f);
+    return make_float2(va ? fb[off(2 * l, i)] : 0.f, vb ? fb[off(2 * l + 1, i)] : 0.f);
   };
   auto store_pair = [&](float *f, int i, float2 v) {
     float *fb = f + base;
@@ -2440,11 +2446,11 @@ static inline void el_go(const SimDev &h, int axis, const ElGrad &g, long long s
   using P = LinePolicy<N>;
   if (axis == 0) {
     using F = typename P::template F<true>;
-    kwb_launch(k_el_grad_fast<F, true, LT, min_ctas<N>(LT)>, cdiv(h.N[1], 2 * LT) * h.N[2], LT * F::G, pline_smem<F>(LT),
+    kwb_launch(k_el_grad_fast<F, true, LT, P::MINB>, cdiv(h.N[1], 2 * LT) * h.N[2], LT * F::G, pline_smem<F>(LT),
                st, h, axis, g, s);
   } else {
     using F = typename P::template F<false>;
-    kwb_launch(k_el_grad_fast<F, false, LT, min_ctas<N>(LT)>, cdiv(h.N[0], 2 * LT) * (axis == 1 ? h.N[2] : h.N[1]),
+    kwb_launch(k_el_grad_fast<F, false, LT, P::MINB>, cdiv(h.N[0], 2 * LT) * (axis == 1 ? h.N[2] : h.N[1]),
                LT * F::G, pline_smem<F>(LT), st, h, axis, g, s);
   }
 }

@@ -85,3 +85,31 @@ def test_reading_a_busy_simulation_holds_up_no_other_thread(other):
     assert np.array_equal(busy.pressure(), field["busy"]) and np.isfinite(field["busy"]).all()
     busy.close()
     idle.close()
+
+
+def elastic_step_us(shape, steps=64, repeats=6):
+    """Device time of one step of a heterogeneous elastic simulation, the best of a few runs."""
+    import kwave_b200 as kb
+    rng = np.random.default_rng(2)
+    g = kb.KWaveGrid(*[v for n in shape for v in (n, 2e-4)])
+    g.dt, g.Nt = 0.3 * 2e-4 / 3200.0, 10 ** 6
+    sim = kb.Simulation(g, kb.ElasticMedium(sound_speed_compression=2600.0 + 600.0 * rng.random(shape),
+                                            sound_speed_shear=1100.0 + 500.0 * rng.random(shape),
+                                            density=1600.0 + 500.0 * rng.random(shape)),
+                        kb.ElasticSource(p0=1e5 * rng.random(shape)), kb.KWaveSensor(), pml_size=10)
+    sim.advance(steps)
+    sim.sync()
+    us = min(sim.advance_timed(steps) for _ in range(repeats)) / steps * 1e3
+    sim.close()
+    return us
+
+
+def test_narrow_elastic_tiles_are_the_faster_ones_where_the_size_rule_takes_them(monkeypatch):
+    """Without a measured schedule (a batch) a 1024^2 elastic grid takes the narrow tiles: 66 us a step, the
+    full-width ones 77.  With too few registers to load its running sums ahead a narrow tile took 81."""
+    monkeypatch.setenv("KWB_TUNE", "0")
+    us = {}
+    for tile in ("big", "small"):
+        monkeypatch.setenv("KWB_TILE", tile)
+        us[tile] = elastic_step_us((1024, 1024))
+    assert us["small"] < 0.97 * us["big"], us
