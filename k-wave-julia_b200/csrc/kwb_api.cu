@@ -243,6 +243,11 @@ bool make_plan_order(int N, FftPlan &pl, int order) {
         break;
       }
   while (r.size() < 2) r.insert(r.begin(), 1);
+  // With a last radix of 16 they fall in the same few banks.  Long lines, whose tiles are one or a few
+  // lines wide, leave a slot free after every 16 positions; below 1024 points the conflicts cost less than
+  // the other instructions do (48 x 40 x 32, whose z passes alone had gaps: 56 -> 59 us a step, most of it in
+  // the pass after them, which had to fetch its code again).
+  pl.sk = N >= 1024 && r.back() == 16 ? 4 : 31;
   int len = N;  // of the sub-transforms at each stage
   for (int R : r) {
     const int st = pl.nstages++;
@@ -387,10 +392,11 @@ std::vector<float2> gradient_conv(const FftPlan &pl, double d, int sign) {
   return spectrum_dif(hk, pl);
 }
 
-int choose_L(int N, int want, int cap_lines) {
+int choose_L(const FftPlan &pl, int want, int cap_lines) {
   int L = want;
   if (L < 1) L = 1;
-  while (L > 1 && line_pass_smem(N, L) > 200 * 1024) L /= 2;
+  // (counted without the gaps between blocks of the last radix, a sixteenth at these lengths)
+  while (L > 1 && (size_t)fft_len(pl) * (lines_pitch(L) + 1) * sizeof(float2) > 200 * 1024) L /= 2;
   if (cap_lines > 0 && L > cap_lines) L = cap_lines;
   if (L < 1) L = 1;
   return L;
@@ -975,7 +981,7 @@ static void sched_store_locked(const std::string &key, const std::string &val) {
 }
 
 // Raised when the step kernels change, so that a file's measurements of older ones are not used.
-#define KWB_SCHED_GEN 3
+#define KWB_SCHED_GEN 4
 
 static std::string sched_key(int device, const SimDev &h) {
   // the device's name, asked once: the query takes 2.5 ms, a sixth of a 128^2 solve of 689 steps
@@ -1176,12 +1182,10 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   // ---- tile shapes and FFT plans
   CU(cudaDeviceGetAttribute(&h.num_sms, cudaDevAttrMultiProcessorCount, ctx->device));
   for (int a = 0; a < 3; ++a) plan_line(h.N[a], h.plan[a], 0);
-  int FL[3];  // transform length per axis (the Bluestein inner length where there is one)
-  for (int a = 0; a < 3; ++a) FL[a] = fft_len(h.plan[a]);
-  h.L_line[0] = choose_L(FL[0], std::max(1, 2048 / h.N[0]), (h.N[1] + 1) / 2);
-  for (int a = 1; a < 3; ++a) h.L_line[a] = choose_L(FL[a], 8, (h.N[0] + 1) / 2);
-  h.L_eosx = choose_L(FL[0], std::max(1, 2048 / h.N[0]), (h.N[1] + 1) / 2);
-  for (int a = 1; a < 3; ++a) h.L_spec[a] = choose_L(FL[a], 8, h.n1);
+  h.L_line[0] = choose_L(h.plan[0], std::max(1, 2048 / h.N[0]), (h.N[1] + 1) / 2);
+  for (int a = 1; a < 3; ++a) h.L_line[a] = choose_L(h.plan[a], 8, (h.N[0] + 1) / 2);
+  h.L_eosx = choose_L(h.plan[0], std::max(1, 2048 / h.N[0]), (h.N[1] + 1) / 2);
+  for (int a = 1; a < 3; ++a) h.L_spec[a] = choose_L(h.plan[a], 8, h.n1);
   h.L_spec[0] = 1;
   {
     // A simulation that runs alone gets narrower tiles and larger CTAs on small grids (latency:

@@ -26,13 +26,18 @@ namespace {
 
 // ---- stages
 
-// The lines in shared memory: position pos of line l at X[pos * PL + l].
+// The lines in shared memory: position pos of line l in slot pos + (pos >> sk), at X[slot * PL + l].
+// The last radix is 2^sk, so that a stage's butterflies still lie a constant number of slots apart: every
+// other stride is a multiple of it.  Without gaps (sk = 31) slot and position are the same; those lengths
+// have code of their own, since the shifts cost them up to 5% (a 1-D step of 243 points 8.5 -> 9.1 us).
+template <bool GAPS>
 struct Lines {
   float2 *X;
   const float2 *tw;
-  int L, PL;
+  int L, PL, sk;
   FastDiv dL;
-  __device__ __forceinline__ float2 &at(int l, int pos) const { return X[pos * PL + l]; }
+  __device__ __forceinline__ int slot(int pos) const { return GAPS ? pos + (pos >> sk) : pos; }
+  __device__ __forceinline__ float2 &at(int l, int pos) const { return X[slot(pos) * PL + l]; }
 };
 
 // call op with the radix as a compile-time constant
@@ -60,15 +65,16 @@ __device__ __forceinline__ void radix_switch(int R, Op &&op) {
 // One stage in place on all lines: butterflies of R slots st positions apart (nb of them over the
 // lines, dst divides by st), twiddle table step ts.  Forward: DFT, then twiddles; backward: conjugate
 // twiddles, then the inverse DFT.
-template <bool INV>
-__device__ __noinline__ void stage(Lines ln, int R_, int st, int ts, int nb, FastDiv dst) {
+template <bool INV, bool GAPS>
+__device__ __noinline__ void stage(Lines<GAPS> ln, int R_, int st, int ts, int nb, FastDiv dst) {
   radix_switch(R_, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
-    const int step = st * ln.PL;
+    if constexpr (R == 1) return;  // (lengths of one stage begin with a 1)
+    const int step = ln.slot(st) * ln.PL;
     for (int b = threadIdx.x; b < nb; b += blockDim.x) {
       const int j = fdiv(b, ln.dL), l = b - j * ln.L;
       const int blk = fdiv(j, dst), u = j - blk * st;
-      float2 *x = ln.X + (blk * st * R + u) * ln.PL + l;
+      float2 *x = ln.X + ln.slot(blk * st * R + u) * ln.PL + l;
       float2 v[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = x[r * step];
@@ -91,12 +97,13 @@ __device__ __noinline__ void stage(Lines ln, int R_, int st, int ts, int nb, Fas
 
 // The last forward stage, the multiply by g (digit-reversed order) and the first backward stage.  A line
 // of one point has radix 1 here too: its transforms are nothing, but g still multiplies it.
-__device__ __noinline__ void stage_top(Lines ln, int R_, int nb, const float2 *__restrict__ g) {
+template <bool GAPS>
+__device__ __noinline__ void stage_top(Lines<GAPS> ln, int R_, int nb, const float2 *__restrict__ g) {
   radix_switch(R_, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
     for (int b = threadIdx.x; b < nb; b += blockDim.x) {
       const int j = fdiv(b, ln.dL), l = b - j * ln.L;
-      float2 *x = ln.X + j * R * ln.PL + l;
+      float2 *x = ln.X + ln.slot(j * R) * ln.PL + l;
       float2 v[R], m[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) m[r] = __ldg(g + j * R + r);
@@ -112,9 +119,8 @@ __device__ __noinline__ void stage_top(Lines ln, int R_, int nb, const float2 *_
   });
 }
 
-template <bool INV>
-__device__ __forceinline__ void run_stage(const Lines &ln, const FftPlan &pl, int s) {
-  if (pl.radix[s] == 1) return;  // (lengths of one stage begin with a 1)
+template <bool INV, bool GAPS>
+__device__ __forceinline__ void run_stage(const Lines<GAPS> &ln, const FftPlan &pl, int s) {
   stage<INV>(ln, pl.radix[s], pl.stride[s], pl.tstride[s], ln.L * pl.nbf[s], pl.div_st[s]);
   __syncthreads();
 }
@@ -122,15 +128,18 @@ __device__ __forceinline__ void run_stage(const Lines &ln, const FftPlan &pl, in
 // Transforms of all lines, natural order <-> digit-reversed order, and circular convolution with the
 // kernel whose transform is g (digit-reversed). The lines are filled before and read after; all
 // threads call them.
-__device__ __forceinline__ void fwd_lines(const Lines &ln, const FftPlan &pl) {
+template <bool GAPS>
+__device__ __forceinline__ void fwd_lines(const Lines<GAPS> &ln, const FftPlan &pl) {
   __syncthreads();
   for (int s = 0; s < pl.nstages; ++s) run_stage<false>(ln, pl, s);
 }
-__device__ __forceinline__ void inv_lines(const Lines &ln, const FftPlan &pl) {
+template <bool GAPS>
+__device__ __forceinline__ void inv_lines(const Lines<GAPS> &ln, const FftPlan &pl) {
   __syncthreads();
   for (int s = pl.nstages - 1; s >= 0; --s) run_stage<true>(ln, pl, s);
 }
-__device__ __forceinline__ void conv_lines(const Lines &ln, const FftPlan &pl, const float2 *g) {
+template <bool GAPS>
+__device__ __forceinline__ void conv_lines(const Lines<GAPS> &ln, const FftPlan &pl, const float2 *g) {
   const int top = pl.nstages - 1;
   __syncthreads();
   for (int s = 0; s < top; ++s) run_stage<false>(ln, pl, s);
@@ -140,7 +149,8 @@ __device__ __forceinline__ void conv_lines(const Lines &ln, const FftPlan &pl, c
 }
 
 // zero the padding of a convolution longer than the line
-__device__ __forceinline__ void clear_tail(const Lines &ln, const FftPlan &pl) {
+template <bool GAPS>
+__device__ __forceinline__ void clear_tail(const Lines<GAPS> &ln, const FftPlan &pl) {
   for (int e = threadIdx.x + pl.n * ln.L; e < pl.m * ln.L; e += blockDim.x) {
     const int pos = fdiv(e, ln.dL);
     ln.at(e - pos * ln.L, pos) = make_float2(0.f, 0.f);
@@ -160,16 +170,18 @@ __device__ __forceinline__ int pos_of(const FftPlan &pl, int k) {
 
 // Dynamic shared memory of a pass: the lines, the twiddles and, for passes that index the spectrum,
 // the digit-reversed position of each frequency (natural order with a convolution in its place).
+template <bool GAPS>
 struct PassSmem {
-  Lines ln;
+  Lines<GAPS> ln;
   unsigned short *at_k;
 };
-__device__ __forceinline__ PassSmem pass_smem(const FftPlan &pl, const float2 *tw_table, int L, FastDiv dL, bool spectrum) {
+template <bool GAPS>
+__device__ __forceinline__ PassSmem<GAPS> pass_smem(const FftPlan &pl, const float2 *tw_table, int L, FastDiv dL, bool spectrum) {
   extern __shared__ float4 smem_raw[];
   const int M = fft_len(pl), PL = lines_pitch(L);
-  float2 *X = reinterpret_cast<float2 *>(smem_raw), *tw = X + M * PL;
+  float2 *X = reinterpret_cast<float2 *>(smem_raw), *tw = X + line_slots(pl) * PL;
   load_twiddles(tw, tw_table, M);
-  PassSmem s{Lines{X, tw, L, PL, dL}, reinterpret_cast<unsigned short *>(tw + M)};
+  PassSmem<GAPS> s{{X, tw, L, PL, pl.sk, dL}, reinterpret_cast<unsigned short *>(tw + M)};
   if (spectrum)
     for (int k = threadIdx.x; k < pl.n; k += blockDim.x)
       s.at_k[k] = (unsigned short)(pl.m > 0 ? k : pl.posof ? __ldg(pl.posof + k) : pos_of(pl, k));
@@ -254,12 +266,12 @@ struct Pairs {
 // Gradient, field update, gradient, field update of one tile of 2L lines.  The first pass of a step
 // (y) waits for the pressure its predecessor wrote; the others load theirs before they wait (as
 // k_line_fast).
-template <bool CONTIG>
+template <bool CONTIG, bool GAPS>
 __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     k_line_pass(const __grid_constant__ SimDev S, int axis, int mode, FastDiv dL, long long step_s) {
   const FftPlan &pl = S.plan[axis];
   const int N = pl.n, L = S.L_line[axis];
-  const Lines ln = pass_smem(pl, S.tw[axis], L, dL, false).ln;
+  const Lines<GAPS> ln = pass_smem<GAPS>(pl, S.tw[axis], L, dL, false).ln;
   const Pairs<CONTIG> pr(S, axis, L);
   const Tile &T = pr.T;
   // point sources on the tile's lines: a thread fetches the entry it will apply ahead of time
@@ -398,12 +410,13 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
 
 // x R2C of [c0^2] rho (1 + Q rho), rho = sum of the split densities, Q = BonA / (2 rho0)
 // (first_order_steps.jl:236-241, 275-279)
+template <bool GAPS>
 __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     k_eos_x_fwd(const __grid_constant__ SimDev S, FastDiv dL, FastDiv dn1, long long step_s) {
   const FftPlan &pl = S.plan[0];
   const int N = pl.n, L = S.L_eosx, n1 = S.n1;
-  const PassSmem sm = pass_smem(pl, S.tw[0], L, dL, true);
-  const Lines &ln = sm.ln;
+  const PassSmem<GAPS> sm = pass_smem<GAPS>(pl, S.tw[0], L, dL, true);
+  const Lines<GAPS> &ln = sm.ln;
   const Pairs<true> pr(S, 0, L);
   KWB_STEP_KERNEL_PROLOGUE();
   if (step_index(S, step_s) >= S.Nt) return;
@@ -447,12 +460,13 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
 }
 
 // x C2R to the pressure (mul_x: 1-D, where no other pass multiplies by M)
+template <bool GAPS>
 __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     k_eos_x_inv(const __grid_constant__ SimDev S, FastDiv dL, FastDiv dn1, long long step_s, int mul_x) {
   const FftPlan &pl = S.plan[0];
   const int N = pl.n, L = S.L_eosx, n1 = S.n1;
-  const PassSmem sm = pass_smem(pl, S.tw[0], L, dL, true);
-  const Lines &ln = sm.ln;
+  const PassSmem<GAPS> sm = pass_smem<GAPS>(pl, S.tw[0], L, dL, true);
+  const Lines<GAPS> &ln = sm.ln;
   const Pairs<true> pr(S, 0, L);
   const bool even = (N & 1) == 0;
   KWB_STEP_KERNEL_PROLOGUE();
@@ -521,12 +535,13 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
 }
 
 // y- or z-direction FFTs of the half spectrum (complex columns kx0..kx0+L-1)
+template <bool GAPS>
 __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     k_spec_pass(const __grid_constant__ SimDev S, int axis, int op, FastDiv dL, long long step_s) {
   const FftPlan &pl = S.plan[axis];
   const int N = pl.n, L = S.L_spec[axis], n1 = S.n1, Ny = S.N[1];
-  const PassSmem sm = pass_smem(pl, S.tw[axis], L, dL, true);
-  const Lines &ln = sm.ln;
+  const PassSmem<GAPS> sm = pass_smem<GAPS>(pl, S.tw[axis], L, dL, true);
+  const Lines<GAPS> &ln = sm.ln;
   const int tpp = (n1 + L - 1) / L;
   const int o = blockIdx.x / tpp;
   const int k0 = (blockIdx.x - o * tpp) * L;
@@ -606,12 +621,12 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
 // ---- elastic gradients
 
 // Directional derivatives of g.nf fields along `axis` on one tile of 2L real lines.
-template <bool CONTIG>
+template <bool CONTIG, bool GAPS>
 __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     k_el_grad(const __grid_constant__ SimDev S, int axis, const __grid_constant__ ElGrad g, FastDiv dL, long long step_s) {
   const FftPlan &pl = S.plan[axis];
   const int N = pl.n, L = S.L_line[axis];
-  const Lines ln = pass_smem(pl, S.tw[axis], L, dL, false).ln;
+  const Lines<GAPS> ln = pass_smem<GAPS>(pl, S.tw[axis], L, dL, false).ln;
   const Pairs<CONTIG> pr(S, axis, L);
   KWB_STEP_KERNEL_PROLOGUE();
   if (step_index(S, step_s) >= S.Nt) return;
@@ -644,12 +659,13 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
 // 5 us each (launch, first loads, tables), 20 us; what bounds it here is the chain of stages and
 // block barriers (about 20) of the three convolutions, 9.4 us.  The steps of a launch keep p, u and
 // rho in shared memory; the medium and the operator tables stay in L1.
+template <bool GAPS>
 __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     k_steps_1d(const __grid_constant__ SimDev S, const __grid_constant__ Groups1D groups, long long t_first, int steps) {
   const FftPlan &pl = S.plan[0];
   const int N = pl.n;
-  const PassSmem sm = pass_smem(pl, S.tw[0], 1, FastDiv{1u, 0u}, true);
-  const Lines &ln = sm.ln;
+  const PassSmem<GAPS> sm = pass_smem<GAPS>(pl, S.tw[0], 1, FastDiv{1u, 0u}, true);
+  const Lines<GAPS> &ln = sm.ln;
   float *P = const_cast<float *>(reinterpret_cast<const float *>(ln.tw + N + (N + 3) / 4));
   float *U = P + N, *Rh = U + N;
   float2 *Prev = reinterpret_cast<float2 *>(P) + (3 * N + 1) / 2;  // dispersion: the last step's spectrum
@@ -759,16 +775,18 @@ __global__ void k_eos1d(float2 *out, const float *M, int N) {
 int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 // a pass that indexes the spectrum also holds the positions
 size_t spectrum_pass_smem(const FftPlan &pl, int L) {
-  return line_pass_smem(fft_len(pl), L) + (size_t)pl.n * sizeof(unsigned short);
+  return line_pass_smem(pl, L) + (size_t)pl.n * sizeof(unsigned short);
 }
 size_t steps1d_smem(const SimDev &h) {
   const int N = h.N[0];
-  return ((size_t)N * lines_pitch(1) + N + (N + 3) / 4 + (3 * N + 1) / 2 + (h.dispersion ? N : 0)) * sizeof(float2);
+  return ((size_t)line_slots(h.plan[0]) * lines_pitch(1) + N + (N + 3) / 4 + (3 * N + 1) / 2 + (h.dispersion ? N : 0)) * sizeof(float2);
 }
 
 }  // namespace
 
-size_t line_pass_smem(int N, int L) { return ((size_t)N * lines_pitch(L) + N) * sizeof(float2); }
+size_t line_pass_smem(const FftPlan &pl, int L) {
+  return ((size_t)line_slots(pl) * lines_pitch(L) + fft_len(pl)) * sizeof(float2);
+}
 
 // Threads per CTA: one butterfly of the first stage each, or, above KWB_PASS_THREADS_MAX of them,
 // equal shares.
@@ -779,72 +797,99 @@ int pass_threads(const FftPlan &pl, int L, int tuned) {
   return std::max(32, ((nb + rounds - 1) / rounds + 31) / 32 * 32);
 }
 
+// op with the kernels of a plan: std::true_type where its lines have gaps
+template <class Op>
+auto by_gaps(const FftPlan &pl, Op &&op) {
+  return pl.sk < 31 ? op(std::true_type{}) : op(std::false_type{});
+}
 cudaError_t generic_prime(const SimDev &h) {
-  cudaError_t e = raise_dynamic_smem((const void *)k_line_pass<true>, line_pass_smem(fft_len(h.plan[0]), h.L_line[0]));
-  size_t line = 0, spec = 0;
-  for (int a = 1; a < h.ndim; ++a) {
-    line = std::max(line, line_pass_smem(fft_len(h.plan[a]), h.L_line[a]));
-    spec = std::max(spec, spectrum_pass_smem(h.plan[a], h.L_spec[a]));
-  }
-  const size_t eos = spectrum_pass_smem(h.plan[0], h.L_eosx);
-  if (e == cudaSuccess) e = raise_dynamic_smem((const void *)k_line_pass<false>, line);
-  if (e == cudaSuccess) e = raise_dynamic_smem((const void *)k_eos_x_fwd, eos);
-  if (e == cudaSuccess) e = raise_dynamic_smem((const void *)k_eos_x_inv, eos);
-  if (e == cudaSuccess) e = raise_dynamic_smem((const void *)k_spec_pass, spec);
+  cudaError_t e = by_gaps(h.plan[0], [&](auto g) {
+    constexpr bool G = decltype(g)::value;
+    cudaError_t e2 = raise_dynamic_smem((const void *)k_line_pass<true, G>, line_pass_smem(h.plan[0], h.L_line[0]));
+    const size_t eos = spectrum_pass_smem(h.plan[0], h.L_eosx);
+    if (e2 == cudaSuccess) e2 = raise_dynamic_smem((const void *)k_eos_x_fwd<G>, eos);
+    return e2 == cudaSuccess ? raise_dynamic_smem((const void *)k_eos_x_inv<G>, eos) : e2;
+  });
+  for (int a = 1; a < h.ndim && e == cudaSuccess; ++a)
+    e = by_gaps(h.plan[a], [&](auto g) {
+      constexpr bool G = decltype(g)::value;
+      const cudaError_t e2 = raise_dynamic_smem((const void *)k_line_pass<false, G>, line_pass_smem(h.plan[a], h.L_line[a]));
+      return e2 == cudaSuccess ? raise_dynamic_smem((const void *)k_spec_pass<G>, spectrum_pass_smem(h.plan[a], h.L_spec[a])) : e2;
+    });
   return e;
 }
 cudaError_t generic_line_pass(const SimDev &h, int axis, int mode, long long step_s, cudaStream_t st) {
   const int L = h.L_line[axis], thr = pass_threads(h.plan[axis], L, h.thr_line[axis]);
-  const size_t sm = line_pass_smem(fft_len(h.plan[axis]), L);
+  const size_t sm = line_pass_smem(h.plan[axis], L);
   const FastDiv dL = make_fastdiv((unsigned)L);
-  if (axis == 0)
-    kwb_launch(k_line_pass<true>, cdiv(h.N[1], 2 * L) * h.N[2], thr, sm, st, h, axis, mode, dL, step_s);
-  else
-    kwb_launch(k_line_pass<false>, cdiv(h.N[0], 2 * L) * (axis == 1 ? h.N[2] : h.N[1]), thr, sm, st, h, axis, mode, dL,
-               step_s);
+  by_gaps(h.plan[axis], [&](auto g) {
+    constexpr bool G = decltype(g)::value;
+    if (axis == 0)
+      kwb_launch(k_line_pass<true, G>, cdiv(h.N[1], 2 * L) * h.N[2], thr, sm, st, h, axis, mode, dL, step_s);
+    else
+      kwb_launch(k_line_pass<false, G>, cdiv(h.N[0], 2 * L) * (axis == 1 ? h.N[2] : h.N[1]), thr, sm, st, h, axis, mode,
+                 dL, step_s);
+  });
   return cudaGetLastError();
 }
 cudaError_t generic_eos(const SimDev &h, bool fwd, long long step_s, cudaStream_t st) {
   const int L = h.L_eosx, grid = cdiv(h.N[1], 2 * L) * h.N[2], thr = pass_threads(h.plan[0], L, 0);
   const size_t sm = spectrum_pass_smem(h.plan[0], L);
   const FastDiv dL = make_fastdiv((unsigned)L), dn1 = make_fastdiv((unsigned)h.n1);
-  if (fwd) kwb_launch(k_eos_x_fwd, grid, thr, sm, st, h, dL, dn1, step_s);
-  else kwb_launch(k_eos_x_inv, grid, thr, sm, st, h, dL, dn1, step_s, h.ndim == 1 ? 1 : 0);
+  by_gaps(h.plan[0], [&](auto g) {
+    constexpr bool G = decltype(g)::value;
+    if (fwd) kwb_launch(k_eos_x_fwd<G>, grid, thr, sm, st, h, dL, dn1, step_s);
+    else kwb_launch(k_eos_x_inv<G>, grid, thr, sm, st, h, dL, dn1, step_s, h.ndim == 1 ? 1 : 0);
+  });
   return cudaGetLastError();
 }
 cudaError_t generic_spec(const SimDev &h, int axis, int op, long long step_s, cudaStream_t st) {
   const int L = h.L_spec[axis];
-  kwb_launch(k_spec_pass, cdiv(h.n1, L) * (axis == 1 ? h.N[2] : h.N[1]), pass_threads(h.plan[axis], L, 0),
-             spectrum_pass_smem(h.plan[axis], L), st, h, axis, op, make_fastdiv((unsigned)L), step_s);
+  by_gaps(h.plan[axis], [&](auto g) {
+    kwb_launch(k_spec_pass<decltype(g)::value>, cdiv(h.n1, L) * (axis == 1 ? h.N[2] : h.N[1]),
+               pass_threads(h.plan[axis], L, 0), spectrum_pass_smem(h.plan[axis], L), st, h, axis, op,
+               make_fastdiv((unsigned)L), step_s);
+  });
   return cudaGetLastError();
 }
 cudaError_t generic_el_prime(const SimDev &h) {
-  size_t m = 0;
-  for (int a = 1; a < h.ndim; ++a) m = std::max(m, line_pass_smem(fft_len(h.plan[a]), h.L_line[a]));
-  const cudaError_t e =
-      raise_dynamic_smem((const void *)k_el_grad<true>, line_pass_smem(fft_len(h.plan[0]), h.L_line[0]));
-  return e != cudaSuccess ? e : raise_dynamic_smem((const void *)k_el_grad<false>, m);
+  cudaError_t e = cudaSuccess;
+  for (int a = 0; a < h.ndim && e == cudaSuccess; ++a)
+    e = by_gaps(h.plan[a], [&](auto g) {
+      constexpr bool G = decltype(g)::value;
+      return raise_dynamic_smem(a == 0 ? (const void *)k_el_grad<true, G> : (const void *)k_el_grad<false, G>,
+                                line_pass_smem(h.plan[a], h.L_line[a]));
+    });
+  return e;
 }
 cudaError_t generic_el_grad(const SimDev &h, int axis, const ElGrad &g, long long s, cudaStream_t st) {
   const int L = h.L_line[axis], thr = pass_threads(h.plan[axis], L, h.thr_line[axis]);
-  const size_t sm = line_pass_smem(fft_len(h.plan[axis]), L);
+  const size_t sm = line_pass_smem(h.plan[axis], L);
   const FastDiv dL = make_fastdiv((unsigned)L);
-  if (axis == 0)
-    kwb_launch(k_el_grad<true>, cdiv(h.N[1], 2 * L) * h.N[2], thr, sm, st, h, axis, g, dL, s);
-  else
-    kwb_launch(k_el_grad<false>, cdiv(h.N[0], 2 * L) * (axis == 1 ? h.N[2] : h.N[1]), thr, sm, st, h, axis, g, dL, s);
+  by_gaps(h.plan[axis], [&](auto gaps) {
+    constexpr bool G = decltype(gaps)::value;
+    if (axis == 0)
+      kwb_launch(k_el_grad<true, G>, cdiv(h.N[1], 2 * L) * h.N[2], thr, sm, st, h, axis, g, dL, s);
+    else
+      kwb_launch(k_el_grad<false, G>, cdiv(h.N[0], 2 * L) * (axis == 1 ? h.N[2] : h.N[1]), thr, sm, st, h, axis, g, dL, s);
+  });
   return cudaGetLastError();
 }
 bool steps1d_fits(const SimDev &h) {
   return h.ndim == 1 && !h.elastic && h.plan[0].m == 0 && steps1d_smem(h) <= 200 * 1024;
 }
-cudaError_t steps1d_prime(const SimDev &h) { return raise_dynamic_smem((const void *)k_steps_1d, steps1d_smem(h)); }
+cudaError_t steps1d_prime(const SimDev &h) {
+  return by_gaps(h.plan[0], [&](auto g) { return raise_dynamic_smem((const void *)k_steps_1d<decltype(g)::value>, steps1d_smem(h)); });
+}
 cudaError_t build_eos1d(float2 *out, const float *M, int N, cudaStream_t st) {
   k_eos1d<<<cdiv(N, 256), 256, 0, st>>>(out, M, N);
   return cudaGetLastError();
 }
 cudaError_t launch_steps1d(const SimDev &h, const Groups1D &g, long long t_first, int steps, cudaStream_t st) {
-  k_steps_1d<<<1, std::max(32, std::min(KWB_PASS_THREADS_MAX, (h.N[0] + 31) / 32 * 32)), steps1d_smem(h), st>>>(h, g, t_first, steps);
+  by_gaps(h.plan[0], [&](auto gaps) {
+    k_steps_1d<decltype(gaps)::value><<<1, std::max(32, std::min(KWB_PASS_THREADS_MAX, (h.N[0] + 31) / 32 * 32)), steps1d_smem(h), st>>>(
+        h, g, t_first, steps);
+  });
   return cudaGetLastError();
 }
 

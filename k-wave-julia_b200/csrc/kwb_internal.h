@@ -62,6 +62,7 @@ struct FftPlan {
   const float2 *chirp_ft;
   const unsigned short *posof;  // digit-reversed position of each frequency (nullptr: worked out)
   FastDiv div_n;  // division by n
+  int sk;         // position pos of a line in shared memory is slot pos + (pos >> sk) (slots of line_slots)
   // per stage: butterflies per line, positions between a butterfly's elements, twiddle-table step,
   // and the divisions by the stride and by the radix
   int nbf[KWB_MAX_STAGES];
@@ -72,6 +73,8 @@ struct FftPlan {
 };
 // Length of the transforms a plan runs (the buffers and twiddle table of a line are this long).
 __host__ __device__ inline int fft_len(const FftPlan &p) { return p.m > 0 ? p.m : p.n; }
+// ... and the slots a line of it takes in shared memory
+__host__ __device__ inline int line_slots(const FftPlan &p) { return fft_len(p) + (fft_len(p) >> p.sk); }
 
 // Pass slots of the FFT schedule: line passes per axis, the x equation-of-state passes, the
 // y/z spectrum passes.
@@ -278,8 +281,8 @@ bool make_plan_order(int N, FftPlan &pl, int order);
 // chirp tables.
 bool plan_line(int N, FftPlan &pl, int order);
 // Complex lines per tile of a pass that fit the shared-memory budget, at most cap_lines (kwb_api.cu).
-int choose_L(int N, int want, int cap_lines);
-size_t line_pass_smem(int N, int L);
+int choose_L(const FftPlan &pl, int want, int cap_lines);
+size_t line_pass_smem(const FftPlan &pl, int L);
 // The passes on the in-place FFTs (kwb_generic.cu); the primes raise their kernels' shared memory.
 struct ElGrad;
 cudaError_t generic_prime(const SimDev &h);

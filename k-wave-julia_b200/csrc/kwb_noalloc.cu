@@ -155,8 +155,8 @@ extern "C" int kwb_eos_pressure_noalloc(int device, int32_t ndim, const int64_t 
   for (int a = 0; a < 3; ++a) h.tw[a] = reinterpret_cast<float2 *>(base + kOffTw + (size_t)a * KWB_MAX_N * 8);
   h.L_line[0] = 1;
   h.L_line[1] = h.L_line[2] = 1;
-  h.L_eosx = choose_L(h.N[0], 2048 / h.N[0], (h.N[1] + 1) / 2);
-  for (int a = 1; a < 3; ++a) h.L_spec[a] = choose_L(h.N[a], 8, h.n1);
+  h.L_eosx = choose_L(h.plan[0], 2048 / h.N[0], (h.N[1] + 1) / 2);
+  for (int a = 1; a < 3; ++a) h.L_spec[a] = choose_L(h.plan[a], 8, h.n1);
   h.Nt = 1;
   h.t0 = reinterpret_cast<long long *>(base + kOffT0);
 

@@ -178,11 +178,11 @@ struct Tuner {
 };
 
 // Lines-per-tile candidates around the heuristic choice L0, clamped as the heuristic is.
-std::vector<int> l_candidates(int N, int L0, int cap) {
+std::vector<int> l_candidates(const FftPlan &pl, int L0, int cap) {
   std::vector<int> out;
   for (int want : {L0, 2 * L0, L0 / 2, L0 / 4}) {
     if (want < 1) continue;
-    const int L = choose_L(N, want, cap);
+    const int L = choose_L(pl, want, cap);
     bool seen = false;
     for (int v : out) seen |= v == L;
     if (!seen) out.push_back(L);
@@ -276,7 +276,7 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
       t.plan[a] = plans[i];
     }, go);
     const int cap = a == 0 ? (t.N[1] + 1) / 2 : (t.N[0] + 1) / 2;
-    const std::vector<int> Ls = l_candidates(fft_len(t.plan[a]), t.L_line[a], cap);
+    const std::vector<int> Ls = l_candidates(t.plan[a], t.L_line[a], cap);
     T.choose("line_L", (int)Ls.size(), [&, a](int i) { t.L_line[a] = Ls[i]; }, go);
     const int thr[4] = {0, 64, 128, 256};
     T.choose("line_threads", 4, [&, a](int i) { t.thr_line[a] = (short)thr[i]; }, go);
@@ -302,7 +302,7 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
       T.choose("eos_inv_tile", 3, [&](int i) { t.tile_var[KWB_SLOT_EOS_INV] = (signed char)i; },
                step);
     } else {
-      const std::vector<int> Ls = l_candidates(fft_len(t.plan[0]), t.L_eosx, (t.N[1] + 1) / 2);
+      const std::vector<int> Ls = l_candidates(t.plan[0], t.L_eosx, (t.N[1] + 1) / 2);
       T.choose("eos_L", (int)Ls.size(), [&](int i) { t.L_eosx = Ls[i]; }, step);
     }
   }
@@ -324,7 +324,7 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
       if (spec_is_fast(t, a)) {
         T.choose("spec_tile", 3, [&, a](int i) { t.tile_var[KWB_SLOT_SPEC1 + a - 1] = (signed char)i; }, go);
       } else {
-        const std::vector<int> Ls = l_candidates(fft_len(t.plan[a]), t.L_spec[a], t.n1);
+        const std::vector<int> Ls = l_candidates(t.plan[a], t.L_spec[a], t.n1);
         T.choose("spec_L", (int)Ls.size(), [&, a](int i) { t.L_spec[a] = Ls[i]; }, go);
       }
     }

@@ -113,3 +113,32 @@ def test_narrow_elastic_tiles_are_the_faster_ones_where_the_size_rule_takes_them
         monkeypatch.setenv("KWB_TILE", tile)
         us[tile] = elastic_step_us((1024, 1024))
     assert us["small"] < 0.97 * us["big"], us
+
+
+# long in-place lines leave a slot free after every 16 positions (last radix 16): 1024 points in 1-D, 2048
+# and 1536 along either axis, one line pair a tile and several, the transforms of a long prime side
+# (1021: length 2048 or more) and the same lengths without gaps in between
+@pytest.mark.parametrize("shape", [(1024,), (2048,), (4096,), (2048, 6), (6, 2048), (1536, 40), (40, 1536), (1021, 9),
+                                   (9, 1021), (2048, 4, 3), (3, 4, 2048), (2000, 9)])
+@pytest.mark.parametrize("stokes", [False, True])
+def test_long_lines_with_gaps(shape, stokes):
+    check(make_case(shape, seed=sum(shape), stokes=stokes, source="p0", steps=30))
+
+
+@pytest.mark.parametrize("shape", [(2048, 12), (12, 2048), (4000, 6), (6, 4096), (1021, 10)])
+def test_elastic_long_lines(shape):
+    import kwave_b200 as kb
+    import kwave_ref as K
+    rng = np.random.Generator(np.random.PCG64(8))
+    cp, cs, rho = (lo + (hi - lo) * rng.random(shape) for lo, hi in ((2600, 3200), (1100, 1600), (1600, 2100)))
+    p0 = 1e5 * rng.random(shape)
+
+    def run(mod):
+        g = mod.KWaveGrid(*[v for n in shape for v in (n, 2e-4)])
+        g.dt, g.Nt = 0.3 * 2e-4 / 3200.0, 25
+        g.t_array = np.arange(25) * g.dt
+        return mod.pstd_elastic_2d(g, mod.ElasticMedium(sound_speed_compression=cp, sound_speed_shear=cs, density=rho),
+                                   mod.ElasticSource(p0=p0),
+                                   mod.KWaveSensor(mask=np.ones(shape, dtype=bool), record=["p_final", "u_max"]), pml_size=2)
+
+    assert_parity(run(kb), run(K), TOL_L2, TOL_MAX)
