@@ -188,12 +188,12 @@ __device__ __forceinline__ PassSmem<GAPS> pass_smem(const FftPlan &pl, const flo
   return s;
 }
 
-// Elements of the tile, UNROLL a thread at a time: load(j, l, i) for each, then use(j, l, i). Element
+// Elements of the tile, UNROLL (or U) a thread at a time: load(j, l, i) for each, then use(j, l, i). Element
 // i of line l; neighbouring lanes take neighbouring positions (BYROW) or lines.  A thread's last
 // round may repeat its first element's load.  (810 x 450 / 120 x 108 x 100, us a step: unrolled once
 // 69.6 / 116.8, twice 66.3 / 112, three times 67.0 / 113.2, four times 68.7 / 113.6, eight 83.7 / 128.)
 constexpr int UNROLL = 2;
-template <bool BYROW, class Load, class Use>
+template <bool BYROW, int U = UNROLL, class Load, class Use>
 __device__ __forceinline__ void elements(int L, int n, FastDiv dL, FastDiv dn, Load &&load, Use &&use) {
   const int total = L * n;
   auto split = [&](int e, int &l, int &i) {
@@ -205,16 +205,16 @@ __device__ __forceinline__ void elements(int L, int n, FastDiv dL, FastDiv dn, L
       l = e - i * L;
     }
   };
-  for (int e0 = threadIdx.x; e0 < total; e0 += UNROLL * blockDim.x) {
+  for (int e0 = threadIdx.x; e0 < total; e0 += U * blockDim.x) {
 #pragma unroll
-    for (int j = 0; j < UNROLL; ++j) {
+    for (int j = 0; j < U; ++j) {
       const int e = e0 + j * (int)blockDim.x;
       int l, i;
       split(e < total ? e : e0, l, i);
       load(j, l, i);
     }
 #pragma unroll
-    for (int j = 0; j < UNROLL; ++j) {
+    for (int j = 0; j < U; ++j) {
       const int e = e0 + j * (int)blockDim.x;
       if (e >= total) break;
       int l, i;
@@ -620,8 +620,10 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
 
 // ---- elastic gradients
 
-// Directional derivatives of g.nf fields along `axis` on one tile of 2L real lines.
-template <bool CONTIG, bool GAPS>
+// Directional derivatives of g.nf fields along `axis` on one tile of 2L real lines, U elements a thread in
+// flight: 8 where a thread has 12 or more (long lines, one or a few a tile), whose sweeps are rounds of
+// memory latency (512 x 2048: 168 -> 153 us a step), 2 elsewhere (60 x 45 with 8: 34 -> 41).
+template <bool CONTIG, bool GAPS, int U>
 __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     k_el_grad(const __grid_constant__ SimDev S, int axis, const __grid_constant__ ElGrad g, FastDiv dL, long long step_s) {
   const FftPlan &pl = S.plan[axis];
@@ -631,16 +633,16 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
   KWB_STEP_KERNEL_PROLOGUE();
   if (step_index(S, step_s) >= S.Nt) return;
   twiddles_landed();
-  float2 a[UNROLL];
+  float2 a[U];
   for (int f = 0; f < g.nf; ++f) {
     const float *src = g.src[f];
     float *dst = g.dst[f];
     const bool acc = (g.acc >> f) & 1;
-    elements<CONTIG>(L, N, dL, pl.div_n, [&](int j, int l, int i) { a[j] = pr.load(src, l, i); },
+    elements<CONTIG, U>(L, N, dL, pl.div_n, [&](int j, int l, int i) { a[j] = pr.load(src, l, i); },
                      [&](int j, int l, int i) { ln.at(l, i) = a[j]; });
     clear_tail(ln, pl);
     conv_lines(ln, pl, S.gdif[axis][g.neg ? 1 : 0]);  // i k e^{+-i k d/2} / N
-    elements<CONTIG>(L, N, dL, pl.div_n,
+    elements<CONTIG, U>(L, N, dL, pl.div_n,
                      [&](int j, int l, int i) { a[j] = acc ? pr.load(dst, l, i) : make_float2(0.f, 0.f); },
                      [&](int j, int l, int i) {
                        const float2 v = ln.at(l, i);
@@ -852,26 +854,49 @@ cudaError_t generic_spec(const SimDev &h, int axis, int op, long long step_s, cu
   });
   return cudaGetLastError();
 }
+// A gradient pass along an axis: CTAs, threads, shared memory, and whether a thread has 12 elements or
+// more of a field (k_el_grad's U).  Long lines of a grid that gives each SM one CTA or two ask for so much
+// shared memory that no SM takes more: launched while the kernel before still runs, they went two and
+// three to the SMs that came free first (4096 x 256, 128 CTAs: 157 -> 109 us a step).
+struct ElPass {
+  int grid, thr;
+  bool deep;
+  size_t smem;
+};
+ElPass el_pass(const SimDev &h, int axis) {
+  const FftPlan &pl = h.plan[axis];
+  const int L = h.L_line[axis];
+  ElPass p;
+  p.grid = axis == 0 ? cdiv(h.N[1], 2 * L) * h.N[2] : cdiv(h.N[0], 2 * L) * (axis == 1 ? h.N[2] : h.N[1]);
+  p.thr = pass_threads(pl, L, h.thr_line[axis]);
+  p.deep = L * pl.n / p.thr >= 12;
+  p.smem = line_pass_smem(pl, L);
+  const int each = cdiv(p.grid, h.num_sms);
+  if (p.deep && each <= 2) p.smem = std::max(p.smem, (size_t)228 * 1024 / (each + 1));
+  return p;
+}
+// op with the kernel of such a pass
+template <class Op>
+auto by_el_kernel(const FftPlan &pl, int axis, bool deep, Op &&op) {
+  return by_gaps(pl, [&](auto g) {
+    constexpr bool G = decltype(g)::value;
+    if (axis == 0) return deep ? op(k_el_grad<true, G, 8>) : op(k_el_grad<true, G, UNROLL>);
+    return deep ? op(k_el_grad<false, G, 8>) : op(k_el_grad<false, G, UNROLL>);
+  });
+}
 cudaError_t generic_el_prime(const SimDev &h) {
   cudaError_t e = cudaSuccess;
-  for (int a = 0; a < h.ndim && e == cudaSuccess; ++a)
-    e = by_gaps(h.plan[a], [&](auto g) {
-      constexpr bool G = decltype(g)::value;
-      return raise_dynamic_smem(a == 0 ? (const void *)k_el_grad<true, G> : (const void *)k_el_grad<false, G>,
-                                line_pass_smem(h.plan[a], h.L_line[a]));
-    });
+  for (int a = 0; a < h.ndim && e == cudaSuccess; ++a) {
+    const ElPass p = el_pass(h, a);
+    e = by_el_kernel(h.plan[a], a, p.deep, [&](auto k) { return raise_dynamic_smem((const void *)k, p.smem); });
+  }
   return e;
 }
 cudaError_t generic_el_grad(const SimDev &h, int axis, const ElGrad &g, long long s, cudaStream_t st) {
-  const int L = h.L_line[axis], thr = pass_threads(h.plan[axis], L, h.thr_line[axis]);
-  const size_t sm = line_pass_smem(h.plan[axis], L);
-  const FastDiv dL = make_fastdiv((unsigned)L);
-  by_gaps(h.plan[axis], [&](auto gaps) {
-    constexpr bool G = decltype(gaps)::value;
-    if (axis == 0)
-      kwb_launch(k_el_grad<true, G>, cdiv(h.N[1], 2 * L) * h.N[2], thr, sm, st, h, axis, g, dL, s);
-    else
-      kwb_launch(k_el_grad<false, G>, cdiv(h.N[0], 2 * L) * (axis == 1 ? h.N[2] : h.N[1]), thr, sm, st, h, axis, g, dL, s);
+  const ElPass p = el_pass(h, axis);
+  by_el_kernel(h.plan[axis], axis, p.deep, [&](auto k) {
+    kwb_launch(k, p.grid, p.thr, p.smem, st, h, axis, g, make_fastdiv((unsigned)h.L_line[axis]), s);
+    return cudaSuccess;
   });
   return cudaGetLastError();
 }
