@@ -1743,9 +1743,21 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   CU(h.elastic ? el_prime(h) : prime_attributes(h));
 
   slog.mark("tr+dense");
-  // ---- FFT schedule: measured on first use of this shape (simulations of the batching
-  // scheduler share the GPU with others, so they keep the heuristic)
-  if (!ctx->batched && S->Nt_loop > 0 && (P->progress || !steps1d_fits(h))) {
+  // ---- 1-D: steps in one launch, unless a callback wants each or there are too many groups to record
+  if (!P->progress && steps1d_fits(h)) {
+    Groups1D &g1 = S->groups1d;
+    int live = 0;
+    for (auto &G : S->groups) {
+      if (G.spec.cartesian || G.n == 0) continue;
+      if (live < KWB_1D_GROUPS) g1.g[live] = G.d_dev;
+      ++live;
+    }
+    g1.n = live;
+    S->steps1d = live <= KWB_1D_GROUPS;
+  }
+  // ---- FFT schedule: measured on first use of this shape where the steps go pass by pass (simulations
+  // of the batching scheduler share the GPU with others, so they keep the heuristic)
+  if (!ctx->batched && S->Nt_loop > 0 && !S->steps1d) {
     if ((rc = choose_schedule(S.get(), h, st))) return rc;
     CU(h.elastic ? el_prime(h) : prime_attributes(h));
     for (int a = 0; a < D; ++a)
@@ -1760,7 +1772,7 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
                             fast_plane_slot_major(h) ? slot_kz : nullptr, st));
   }
 
-  if (D == 1 && steps1d_fits(h)) {
+  if (S->steps1d) {
     const int n = h.N[0];
     float2 *nat, *op;
     CU(M.alloc(&nat, n));
@@ -1768,6 +1780,7 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
     CU(build_eos1d(nat, h.M, n, st));
     CU(permute_dif(op, nat, h.plan[0], st));
     h.eos1d = op;
+    CU(steps1d_prime(h));
   }
 
   slog.mark("schedule");
@@ -1791,20 +1804,6 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   S->progress = P->progress;
   S->progress_user = P->progress_user;
   if (S->progress) CU(cudaMallocHost(&S->p_host, nvox * 4));
-  if (!S->progress && steps1d_fits(h)) {
-    Groups1D &g1 = S->groups1d;
-    int live = 0;
-    for (auto &G : S->groups) {
-      if (G.spec.cartesian || G.n == 0) continue;
-      if (live < KWB_1D_GROUPS) g1.g[live] = G.d_dev;
-      ++live;
-    }
-    g1.n = live;
-    if (live <= KWB_1D_GROUPS) {
-      CU(steps1d_prime(h));
-      S->steps1d = true;
-    }
-  }
   S->launches_per_step = count_launches(S.get());
   slog.done();
   *out = S.release();

@@ -142,3 +142,29 @@ def test_elastic_long_lines(shape):
                                    mod.KWaveSensor(mask=np.ones(shape, dtype=bool), record=["p_final", "u_max"]), pml_size=2)
 
     assert_parity(run(kb), run(K), TOL_L2, TOL_MAX)
+
+
+def test_a_line_with_many_sensor_groups_has_a_measured_schedule(monkeypatch, tmp_path):
+    """More than eight recorded groups go pass by pass, with the schedule of their shape measured; eight run
+    in one launch.  Every group records the same."""
+    import kwave_b200 as kb
+    for k in ("KWB_TUNE", "KWB_TUNE_PICK", "KWB_TUNE_ORDER", "KWB_TILE"):
+        monkeypatch.delenv(k, raising=False)
+    n = 1100
+    case = make_case((n,), source="p0", steps=40)
+    g, m, s, _, kw = case.to_api()
+    mask = np.zeros(n, dtype=bool)
+    mask[3::7] = True
+    sensor = kb.KWaveSensor(mask=mask, record=["p_max", "p_final"])
+    outs = []
+    for extra, launches, src in ((7, 1, "heuristic"), (8, 12, "tuned")):
+        sim = kb.Simulation(g, m, s, sensor, extra_sensors=[sensor] * extra, **kw)
+        assert sim.info()["launches_per_step"] == launches
+        assert sim.schedule().startswith(src) or sim.schedule().startswith("cache") and src == "tuned", sim.schedule()
+        sim.advance(sim.Nt)
+        outs.append(sim.outputs())
+        assert len(outs[-1].extra) == extra
+        for group in outs[-1].extra:
+            assert all(np.array_equal(group[f], outs[-1][f]) for f in ("p_max", "p_final"))
+        sim.close()
+    assert_parity(outs[1], outs[0], TOL_L2, TOL_MAX)
