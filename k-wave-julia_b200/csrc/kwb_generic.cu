@@ -820,22 +820,30 @@ cudaError_t generic_prime(const SimDev &h) {
     });
   return e;
 }
+// ... of a fluid pass: where it has at most two tiles an SM and the simulation runs alone, at least a
+// thread for every 4 elements, since its sweeps are then rounds of memory latency (us a step without a
+// measured schedule: 112^2 61 -> 52, 30 x 64 37.8 -> 32.4, 270 x 256 63.7 -> 45.9, 810 x 450 75 -> 71);
+// in larger grids, which hide it, more threads leave room for fewer CTAs (120 x 108 x 100 128 -> 141).
+static int fluid_threads(const SimDev &h, int axis, int L, int grid, int tuned) {
+  const int thr = pass_threads(h.plan[axis], L, tuned);
+  if (tuned > 0 || !h.grid_fill || grid > 2 * h.num_sms) return thr;
+  return std::max(thr, std::min(KWB_PASS_THREADS_MAX, (L * h.plan[axis].n / 4 + 31) / 32 * 32));
+}
 cudaError_t generic_line_pass(const SimDev &h, int axis, int mode, long long step_s, cudaStream_t st) {
-  const int L = h.L_line[axis], thr = pass_threads(h.plan[axis], L, h.thr_line[axis]);
+  const int L = h.L_line[axis];
+  const int grid = axis == 0 ? cdiv(h.N[1], 2 * L) * h.N[2] : cdiv(h.N[0], 2 * L) * (axis == 1 ? h.N[2] : h.N[1]);
+  const int thr = fluid_threads(h, axis, L, grid, h.thr_line[axis]);
   const size_t sm = line_pass_smem(h.plan[axis], L);
   const FastDiv dL = make_fastdiv((unsigned)L);
   by_gaps(h.plan[axis], [&](auto g) {
     constexpr bool G = decltype(g)::value;
-    if (axis == 0)
-      kwb_launch(k_line_pass<true, G>, cdiv(h.N[1], 2 * L) * h.N[2], thr, sm, st, h, axis, mode, dL, step_s);
-    else
-      kwb_launch(k_line_pass<false, G>, cdiv(h.N[0], 2 * L) * (axis == 1 ? h.N[2] : h.N[1]), thr, sm, st, h, axis, mode,
-                 dL, step_s);
+    if (axis == 0) kwb_launch(k_line_pass<true, G>, grid, thr, sm, st, h, axis, mode, dL, step_s);
+    else kwb_launch(k_line_pass<false, G>, grid, thr, sm, st, h, axis, mode, dL, step_s);
   });
   return cudaGetLastError();
 }
 cudaError_t generic_eos(const SimDev &h, bool fwd, long long step_s, cudaStream_t st) {
-  const int L = h.L_eosx, grid = cdiv(h.N[1], 2 * L) * h.N[2], thr = pass_threads(h.plan[0], L, 0);
+  const int L = h.L_eosx, grid = cdiv(h.N[1], 2 * L) * h.N[2], thr = fluid_threads(h, 0, L, grid, 0);
   const size_t sm = spectrum_pass_smem(h.plan[0], L);
   const FastDiv dL = make_fastdiv((unsigned)L), dn1 = make_fastdiv((unsigned)h.n1);
   by_gaps(h.plan[0], [&](auto g) {
@@ -846,11 +854,10 @@ cudaError_t generic_eos(const SimDev &h, bool fwd, long long step_s, cudaStream_
   return cudaGetLastError();
 }
 cudaError_t generic_spec(const SimDev &h, int axis, int op, long long step_s, cudaStream_t st) {
-  const int L = h.L_spec[axis];
+  const int L = h.L_spec[axis], grid = cdiv(h.n1, L) * (axis == 1 ? h.N[2] : h.N[1]);
   by_gaps(h.plan[axis], [&](auto g) {
-    kwb_launch(k_spec_pass<decltype(g)::value>, cdiv(h.n1, L) * (axis == 1 ? h.N[2] : h.N[1]),
-               pass_threads(h.plan[axis], L, 0), spectrum_pass_smem(h.plan[axis], L), st, h, axis, op,
-               make_fastdiv((unsigned)L), step_s);
+    kwb_launch(k_spec_pass<decltype(g)::value>, grid, fluid_threads(h, axis, L, grid, 0),
+               spectrum_pass_smem(h.plan[axis], L), st, h, axis, op, make_fastdiv((unsigned)L), step_s);
   });
   return cudaGetLastError();
 }

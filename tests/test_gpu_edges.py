@@ -168,3 +168,20 @@ def test_a_line_with_many_sensor_groups_has_a_measured_schedule(monkeypatch, tmp
             assert all(np.array_equal(group[f], outs[-1][f]) for f in ("p_max", "p_final"))
         sim.close()
     assert_parity(outs[1], outs[0], TOL_L2, TOL_MAX)
+
+
+def test_the_size_rule_of_a_small_grid_is_near_its_measured_schedule(monkeypatch):
+    """270 x 256 without a measured schedule: 46 us a step against 45 with one.  With a thread per first-stage
+    butterfly alone its strided passes had 10 elements a thread in rounds of memory latency: 64."""
+    import kwave_b200 as kb
+    for k in ("KWB_TUNE_PICK", "KWB_TUNE_ORDER", "KWB_TILE"):
+        monkeypatch.delenv(k, raising=False)
+    us = {}
+    for tune in ("0", "1"):
+        monkeypatch.setenv("KWB_TUNE", tune)
+        g, m, s, sen, kw = make_case((270, 256), source="p0", record=("p_max",), steps=2000).to_api()
+        sim = kb.Simulation(g, m, s, kb.KWaveSensor(), **kw)
+        sim.advance(64)
+        us[tune] = min(sim.advance_timed(64) for _ in range(6)) / 64 * 1e3
+        sim.close()
+    assert us["0"] < 1.2 * us["1"], us
