@@ -12,13 +12,17 @@
 //   * the elastic solver's gradient passes: the tile variant of each axis.
 // Each candidate runs on the simulation's own buffers before its initial conditions are set
 // (sensors, sources and time reversal are switched off in the timing descriptor): one warm-up
-// time step, then three timed with CUDA events (on grids of up to 4 Mi points a replayed graph of
-// 16 steps, as the simulation runs them), so that a candidate is judged by the step it gives; the passes are tuned one at a time, each with the others at their current choice.  Every candidate computes the same transform: the tile shape
+// time step, then three timed with CUDA events (on grids of up to 4 Mi points a replayed graph, as
+// the simulation runs them), so that a candidate is judged by the step it gives; the passes are tuned
+// one at a time, each with the others at their current choice.  Every candidate computes the same
+// transform: the tile shape
 // and thread count leave the arithmetic of each line unchanged, so results are bit-identical
 // whatever is picked -- a simulation gives the same fields alone, tuned, and in a batch, which
 // keeps the heuristic.  A different radix order only reorders FP32 rounding; it is explored
 // only on request (KWB_TUNE_ORDER=1), since it gives up that bit-for-bit agreement.
+#include <algorithm>
 #include <cfloat>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -114,40 +118,52 @@ struct Tuner {
   // Average device time of one launch of `go` (a time step) with the descriptor t (FLT_MAX if it
   // failed).  Grids whose steps take tens of microseconds are timed as their simulation runs them,
   // from a replayed graph: launched one by one, a 512^2 step took the host's 20 us whatever its
-  // tiles, and the choice was left to noise (128^2: 15.0 or 18.2 us a step).
+  // tiles, and the choice was left to noise (128^2: 15.0 or 18.2 us a step).  The graph holds 4
+  // steps, is replayed once as a warm-up and then for a quarter of a millisecond, at least once and
+  // at most 4 times: 9 to 21 steps a candidate, what the first simulation of a shape waits for.
   template <class F>
   float time(F go) {
     cudaError_t e = cudaMemcpyAsync(d_t, &t, sizeof(SimDev), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = t.elastic ? el_prime(t) : prime_attributes(t);
     if (e == cudaSuccess) e = go();
-    const int reps = t.nvox <= (4LL << 20) ? 16 : 3;
+    constexpr int kGraphSteps = 4;
+    const bool replay = t.nvox <= (4LL << 20);
     cudaGraphExec_t ex = nullptr;
-    if (reps > 3 && e == cudaSuccess) {
+    if (replay && e == cudaSuccess) {
       cudaGraph_t g = nullptr;
       e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-      for (int r = 0; r < reps && e == cudaSuccess; ++r) e = go();
+      for (int r = 0; r < kGraphSteps && e == cudaSuccess; ++r) e = go();
       const cudaError_t e2 = cudaStreamEndCapture(st, &g);
       if (e == cudaSuccess) e = e2;
       if (e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
       if (g) cudaGraphDestroy(g);
-      if (e == cudaSuccess) e = cudaGraphLaunch(ex, st);
     }
-    if (e == cudaSuccess) e = cudaEventRecord(e0, st);
-    if (ex && e == cudaSuccess) e = cudaGraphLaunch(ex, st);
-    for (int r = 0; !ex && r < reps && e == cudaSuccess; ++r) e = go();
-    if (e == cudaSuccess) e = cudaEventRecord(e1, st);
-    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+    // `n` runs of `once` between two events: milliseconds
+    auto span = [&](int n, auto once) -> float {
+      float ms = 0.f;
+      if (e == cudaSuccess) e = cudaEventRecord(e0, st);
+      for (int r = 0; r < n && e == cudaSuccess; ++r) e = once();
+      if (e == cudaSuccess) e = cudaEventRecord(e1, st);
+      if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+      return ms;
+    };
+    float ms;
     if (ex) {
+      auto once = [&] { return cudaGraphLaunch(ex, st); };
+      const float warm = span(1, once);
+      const int n = std::max(1, std::min(4, (int)std::ceil(0.25f / std::max(warm, 1e-3f))));
+      ms = span(n, once) / (float)(n * kGraphSteps);
       cudaStreamSynchronize(st);
       cudaGraphExecDestroy(ex);
+    } else {
+      ms = span(3, go) / 3.f;
     }
-    float ms = 0.f;
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return FLT_MAX;
     }
-    return ms / (float)reps;
+    return ms;
   }
 
   // Try `n` candidates set by set(i) (i < n), keep the fastest (or candidate `pick`).

@@ -185,3 +185,30 @@ def test_the_size_rule_of_a_small_grid_is_near_its_measured_schedule(monkeypatch
         us[tune] = min(sim.advance_timed(64) for _ in range(6)) / 64 * 1e3
         sim.close()
     assert us["0"] < 1.2 * us["1"], us
+
+
+def test_the_first_simulation_of_a_shape_waits_for_few_steps(monkeypatch):
+    """What measuring the schedule of a shape costs, in time steps of it: 24 candidates of 9 steps each at
+    100 x 98 x 96 elastic, and the capture of their graphs.  With 33 steps a candidate it was 1000."""
+    import time
+    for k in ("KWB_TUNE", "KWB_TUNE_PICK", "KWB_TUNE_ORDER", "KWB_TILE"):
+        monkeypatch.delenv(k, raising=False)
+    import kwave_b200 as kb
+    shape = (100, 98, 96)
+    rng = np.random.default_rng(4)
+    g = kb.KWaveGrid(*[v for n in shape for v in (n, 2e-4)])
+    g.dt, g.Nt = 0.3 * 2e-4 / 3200.0, 10 ** 6
+    med = kb.ElasticMedium(sound_speed_compression=2600.0 + 600.0 * rng.random(shape),
+                           sound_speed_shear=1100.0 + 500.0 * rng.random(shape), density=1600.0 + 500.0 * rng.random(shape))
+    took = []
+    for _ in range(3):
+        t = time.perf_counter()
+        sim = kb.Simulation(g, med, kb.ElasticSource(), kb.KWaveSensor(), pml_size=10)
+        took.append(time.perf_counter() - t)
+        if len(took) < 3:
+            sim.close()
+    assert sim.schedule().startswith("cache")
+    sim.advance(32)
+    step = min(sim.advance_timed(32) for _ in range(4)) / 32 * 1e-3
+    sim.close()
+    assert took[0] - min(took[1:]) < 500 * step, (took, step)
