@@ -212,3 +212,20 @@ def test_the_first_simulation_of_a_shape_waits_for_few_steps(monkeypatch):
     step = min(sim.advance_timed(32) for _ in range(4)) / 32 * 1e-3
     sim.close()
     assert took[0] - min(took[1:]) < 500 * step, (took, step)
+
+
+def test_tables_of_a_long_prime_side_do_not_dominate_its_set_up():
+    """Creating a 1-D simulation of 2039 points (a prime: three tables of 4096-point transforms) against one
+    of 2048.  With the tables summed term by term: 10 ms against 0.8."""
+    import time
+    import kwave_b200 as kb
+    ms = {}
+    for n in (2039, 2048):
+        g, m, s, _, kw = make_case((n,), source="p0", steps=20).to_api()
+        ms[n] = 1e9
+        for _ in range(6):
+            t = time.perf_counter()
+            sim = kb.Simulation(g, m, s, kb.KWaveSensor(), **kw)
+            ms[n] = min(ms[n], 1e3 * (time.perf_counter() - t))
+            sim.close()
+    assert ms[2039] < 4 * ms[2048], ms
