@@ -780,6 +780,7 @@ cudaError_t enqueue_step(kwb_sim *S, long long step_s) {
     if ((e = launch_line_pass(S->d_sim, h, a, KWB_MODE_STEP, step_s, st)) != cudaSuccess) return e;
   }
   if (!h.fuse_xeos && (e = launch_eos_x_fwd(S->d_sim, h, step_s, st)) != cudaSuccess) return e;
+  if ((e = launch_change_spectrum(h, step_s, st)) != cudaSuccess) return e;
   if (h.ndim == 2) {
     if ((e = launch_spec_pass(S->d_sim, h, 1, KWB_SPEC_FWD_MUL_INV, step_s, st)) != cudaSuccess) return e;
   } else if (h.ndim == 3 && h.plane) {
@@ -805,13 +806,47 @@ int count_launches(const kwb_sim *S) {
       if (!g.spec.cartesian && g.n > 0) ++n;
     return n;
   }
-  int n = (S->tr ? 1 : 0) + S->h.ndim + (S->h.fuse_xeos ? 1 : 2) + (S->h.ndim == 2 ? 1 : (S->h.ndim == 3 ? (S->h.plane ? 1 : 3) : 0));
+  int n = (S->tr ? 1 : 0) + S->h.ndim + (S->h.fuse_xeos ? 1 : 2) + (S->h.ndim == 2 ? 1 : (S->h.ndim == 3 ? (S->h.plane ? 1 : 3) : 0)) + change_launches(S->h);
   for (auto &g : S->groups)
     if (!g.spec.cartesian && g.n > 0 && !g.fused) ++n;
   return n;
 }
 
 }  // namespace
+
+// Factors of an absorbing medium (solver/first_order.jl:13-42), c the reference sound speed.
+struct Absorption {
+  double tau, eta, y;
+};
+static Absorption absorption_of(const kwb_problem *P, double c) {
+  const double y = P->alpha_power;
+  const double a_np = P->alpha_coeff * (1e-2 / (20.0 * std::log10(std::exp(1.0)))) * std::pow(2.0 * kPi * 1e6, -y);
+  return Absorption{-2.0 * a_np * std::pow(c, y - 1.0), 2.0 * a_np * std::pow(c, y - 1.0) * std::tan(kPi * y / 2.0), y};
+}
+
+// How a simulation takes the dispersion term (scalar c0 with :stokes): from the last step's spectrum, which
+// costs no transform, while the term's multiplier eta k^(y-1) / dt stays below a tenth of the equation of
+// state's own, 1 + tau k^y, at the longest and the shortest wave of the grid; above, where the rounding
+// of the two full spectra would outweigh that of everything else (error over 120 steps at 64 x 96, dx = 1e-5,
+// CFL 0.1, y = 1.5, a ratio of 4: 4.6e-7 against 2.2e-7; at 0.05 and 0.1 they are the same within 8%), from a
+// transform of the change.
+static int dispersion_mode(const kwb_problem *P, long long nvox) {
+  if (P->elastic || P->alpha_mode != KWB_STOKES || (P->c0.count == nvox && nvox > 1)) return KWB_DISP_NONE;
+  if (P->c0.count < 1 || !P->c0.data) return KWB_DISP_LAST;  // (an estimate for a problem not yet looked over)
+  const Absorption ab = absorption_of(P, P->c0.data[0]);
+  double k_min = INFINITY, k_max2 = 0.0;
+  for (int a = 0; a < P->ndim; ++a) {
+    if (P->N[a] < 2) continue;
+    k_min = std::min(k_min, 2.0 * kPi / ((double)P->N[a] * P->d[a]));
+    k_max2 += (kPi / P->d[a]) * (kPi / P->d[a]);
+  }
+  if (k_max2 == 0.0) return KWB_DISP_LAST;  // a grid of one point: the mean alone
+  for (double k : {k_min, std::sqrt(k_max2)}) {
+    const double own = 1.0 + ab.tau * std::pow(k, ab.y);
+    if (!(std::fabs(ab.eta * std::pow(k, ab.y - 1.0) / P->dt) <= 0.1 * own)) return KWB_DISP_CHANGE;
+  }
+  return KWB_DISP_LAST;
+}
 
 // Device bytes a simulation of `P` holds (fields, spectra, medium, tables, sensor buffers and
 // the FP64 upload staging), the figure admission control compares with free memory.
@@ -825,7 +860,7 @@ size_t estimate_device_bytes(const kwb_problem *P) {
   const bool r_arr = P->rho0.count == nvox && nvox > 1;
   const bool b_arr = P->BonA.count == nvox && nvox > 1;
   const bool nonlinear = P->BonA.count > 0;
-  const bool dispersion = !c_arr && P->alpha_mode == KWB_STOKES && !P->elastic;
+  const int dispersion = dispersion_mode(P, nvox);
   size_t need;
   if (P->elastic) {
     // p, velocities, stresses and derivative scratch; rho0, lambda and mu per voxel with an array
@@ -838,7 +873,7 @@ size_t estimate_device_bytes(const kwb_problem *P) {
     need += (size_t)P->n_s_index * 8 + (size_t)P->n_u_index * 8;
   } else {
     need = (size_t)nvox * 4 * (1 + 2 * D) + (size_t)nspec * 8;
-    if (dispersion) need += (size_t)nspec * 8;
+    if (dispersion) need += (size_t)nspec * 8 + (dispersion == KWB_DISP_CHANGE ? (size_t)nvox * 4 : 0);
     need += (size_t)nspec * 4 * (dispersion ? 2 : 1);
     need += (size_t)nvox * 4 * ((r_arr ? 1 : 0) + (c_arr ? 1 : 0) + ((nonlinear && (b_arr || r_arr)) ? 1 : 0));
     // FP64 staging during set-up (released once the simulation is created)
@@ -1060,6 +1095,7 @@ static int choose_schedule(kwb_sim *S, SimDev &h, cudaStream_t st) {
     if (f) CU(cudaMemsetAsync(f, 0, nvox * 4, st));
   if (h.spec) CU(cudaMemsetAsync(h.spec, 0, h.nspec * sizeof(float2), st));
   if (h.spec2) CU(cudaMemsetAsync(h.spec2, 0, h.nspec * sizeof(float2), st));
+  if (h.rho_prev) CU(cudaMemsetAsync(h.rho_prev, 0, nvox * 4, st));
   schedule_of(h, sc);
   if (pick >= 0) {
     S->schedule_src = "pick " + std::to_string(pick);
@@ -1160,17 +1196,16 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   const bool nonlinear = P->BonA.count > 0;
   h.nonlinear = nonlinear;
   h.scalar_c = !c_arr;
-  h.dispersion = (!c_arr && absorbing && P->alpha_mode == KWB_STOKES && !h.elastic) ? 1 : 0;
+  h.dispersion = dispersion_mode(P, nvox);
   h.dt_over_rho0_s = (float)(P->dt / r_s);
   h.dt_rho0_s = (float)(P->dt * r_s);
   h.c0sq_s = (float)(c_s * c_s);
   double tau = 0, eta = 0, y = 0;
   if (absorbing) {
-    y = P->alpha_power;
-    const double a_np = P->alpha_coeff * (1e-2 / (20.0 * std::log10(std::exp(1.0)))) *
-                        std::pow(2.0 * kPi * 1e6, -y);
-    tau = -2.0 * a_np * std::pow(c_ref, y - 1.0);
-    eta = 2.0 * a_np * std::pow(c_ref, y - 1.0) * std::tan(kPi * y / 2.0);
+    const Absorption ab = absorption_of(P, c_ref);
+    tau = ab.tau;
+    eta = ab.eta;
+    y = ab.y;
   }
 
   // ---- FFT path: register-FFT kernels for power-of-two lines unless KWB_FFT_PATH=generic
@@ -1273,6 +1308,10 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
   if (h.dispersion) {
     CU(M.alloc(&h.spec2, h.nspec));  // the spectrum of the step before: none yet (rho_prev = 0)
     CU(cudaMemsetAsync(h.spec2, 0, h.nspec * sizeof(float2), st));
+  }
+  if (h.dispersion == KWB_DISP_CHANGE) {
+    CU(M.alloc(&h.rho_prev, nvox));
+    CU(cudaMemsetAsync(h.rho_prev, 0, nvox * 4, st));
   }
   CU(M.alloc(&S->d_t0, 1));
   CU(cudaMemsetAsync(S->d_t0, 0, 8, st));
@@ -1779,7 +1818,7 @@ int kwb_sim_create(kwb_ctx *ctx, const kwb_problem *P, kwb_sim **out) {
     const double d3[3] = {P->d[0], D > 1 ? P->d[1] : 1.0, D > 2 ? P->d[2] : 1.0};
     CU(build_eos_multiplier(const_cast<float *>(h.M), const_cast<float *>(h.M2), h.N, d3, c_ref, P->dt,
                             c_arr ? 1.0 : c_s * c_s, absorbing, tau, eta, y, h.plane ? slot_ky : nullptr,
-                            fast_plane_slot_major(h) ? slot_kz : nullptr, st));
+                            fast_plane_slot_major(h) ? slot_kz : nullptr, h.dispersion, st));
   }
 
   if (S->steps1d) {
@@ -2235,6 +2274,8 @@ int kwb_sim_profile(kwb_sim *S, int64_t steps, kwb_kernel_times *out) {
     }
     if (!h.fuse_xeos)
       timed(slot("eos_x_fwd", eos_rd + ns * 8.0), [&] { return launch_eos_x_fwd(S->d_sim, h, s, st); });
+    if (change_launches(h))
+      timed(slot("change_spectrum", eos_rd + nv * 8.0 + ns * (16.0 * h.ndim - 8.0)), [&] { return launch_change_spectrum(h, s, st); });
     if (h.ndim == 2) {
       timed(slot("spec_y_mul", ns * 8.0 * (h.dispersion ? 4 : 2) + ns * 4.0 * (h.dispersion ? 2 : 1)),
             [&] { return launch_spec_pass(S->d_sim, h, 1, KWB_SPEC_FWD_MUL_INV, s, st); });

@@ -409,8 +409,9 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
 // ---- equation of state
 
 // x R2C of [c0^2] rho (1 + Q rho), rho = sum of the split densities, Q = BonA / (2 rho0)
-// (first_order_steps.jl:236-241, 275-279)
-template <bool GAPS>
+// (first_order_steps.jl:236-241, 275-279); CHANGE: of its change since the last step
+// (first_order_steps.jl:255-263, 436-440)
+template <bool GAPS, bool CHANGE>
 __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     k_eos_x_fwd(const __grid_constant__ SimDev S, FastDiv dL, FastDiv dn1, long long step_s) {
   const FftPlan &pl = S.plan[0];
@@ -437,6 +438,11 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
         if (S.D > 2) v = cadd(v, c[j]);
         if (S.nonlinear) v = make_float2(v.x * fmaf(q[j].x, v.x, 1.0f), v.y * fmaf(q[j].y, v.y, 1.0f));
         if (S.c0sq) v = make_float2(w[j].x * v.x, w[j].y * v.y);
+        if (CHANGE) {  // since the last step
+          const float2 r = v;
+          v = csub(v, pr.load(S.rho_prev, l, i));
+          pr.store(S.rho_prev, l, i, r);
+        }
         ln.at(l, i) = pl.m > 0 ? cmul(v, __ldg(pl.chirp + i)) : v;
       });
   clear_tail(ln, pl);
@@ -479,7 +485,7 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
       if (S.dispersion) {  // the spectrum of the step before (build_eos_multiplier)
         const float m2 = S.M2[q * n1 + k];
         const float2 b = __ldcg(S.spec2 + q * n1 + k);
-        S.spec2[q * n1 + k] = v;
+        if (S.dispersion == KWB_DISP_LAST) S.spec2[q * n1 + k] = v;
         v = make_float2(fmaf(m2, b.x, m * v.x), fmaf(m2, b.y, m * v.y));
       } else {
         v = cscale(v, m);
@@ -581,7 +587,7 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
   }
   if (op == KWB_SPEC_FWD_MUL_INV) {
     // the equation of state: times M, and with dispersion plus M2 times the spectrum of the step
-    // before, which this pass keeps in spec2 (build_eos_multiplier)
+    // before, which this pass keeps in spec2, or of the change since (build_eos_multiplier)
     elements<false>(
         L, N, dL, pl.div_n,
         [&](int j, int l, int k) {
@@ -596,7 +602,7 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
           const float2 w = blue ? __ldg(pl.chirp + k) : zero;
           if (blue) z = cmul(z, w);
           if (S.dispersion) {
-            if (l < cnt) S.spec2[at(l, k)] = z;
+            if (l < cnt && S.dispersion == KWB_DISP_LAST) S.spec2[at(l, k)] = z;
             z = make_float2(fmaf(m2[j], b[j].x, m[j] * z.x), fmaf(m2[j], b[j].y, m[j] * z.y));
           } else {
             z = cscale(z, m[j]);
@@ -809,7 +815,8 @@ cudaError_t generic_prime(const SimDev &h) {
     constexpr bool G = decltype(g)::value;
     cudaError_t e2 = raise_dynamic_smem((const void *)k_line_pass<true, G>, line_pass_smem(h.plan[0], h.L_line[0]));
     const size_t eos = spectrum_pass_smem(h.plan[0], h.L_eosx);
-    if (e2 == cudaSuccess) e2 = raise_dynamic_smem((const void *)k_eos_x_fwd<G>, eos);
+    if (e2 == cudaSuccess) e2 = raise_dynamic_smem((const void *)k_eos_x_fwd<G, false>, eos);
+    if (e2 == cudaSuccess) e2 = raise_dynamic_smem((const void *)k_eos_x_fwd<G, true>, eos);
     return e2 == cudaSuccess ? raise_dynamic_smem((const void *)k_eos_x_inv<G>, eos) : e2;
   });
   for (int a = 1; a < h.ndim && e == cudaSuccess; ++a)
@@ -842,13 +849,14 @@ cudaError_t generic_line_pass(const SimDev &h, int axis, int mode, long long ste
   });
   return cudaGetLastError();
 }
-cudaError_t generic_eos(const SimDev &h, bool fwd, long long step_s, cudaStream_t st) {
+cudaError_t generic_eos(const SimDev &h, bool fwd, long long step_s, cudaStream_t st, bool change) {
   const int L = h.L_eosx, grid = cdiv(h.N[1], 2 * L) * h.N[2], thr = fluid_threads(h, 0, L, grid, 0);
   const size_t sm = spectrum_pass_smem(h.plan[0], L);
   const FastDiv dL = make_fastdiv((unsigned)L), dn1 = make_fastdiv((unsigned)h.n1);
   by_gaps(h.plan[0], [&](auto g) {
     constexpr bool G = decltype(g)::value;
-    if (fwd) kwb_launch(k_eos_x_fwd<G>, grid, thr, sm, st, h, dL, dn1, step_s);
+    if (fwd && change) kwb_launch(k_eos_x_fwd<G, true>, grid, thr, sm, st, h, dL, dn1, step_s);
+    else if (fwd) kwb_launch(k_eos_x_fwd<G, false>, grid, thr, sm, st, h, dL, dn1, step_s);
     else kwb_launch(k_eos_x_inv<G>, grid, thr, sm, st, h, dL, dn1, step_s, h.ndim == 1 ? 1 : 0);
   });
   return cudaGetLastError();
@@ -908,7 +916,7 @@ cudaError_t generic_el_grad(const SimDev &h, int axis, const ElGrad &g, long lon
   return cudaGetLastError();
 }
 bool steps1d_fits(const SimDev &h) {
-  return h.ndim == 1 && !h.elastic && h.plan[0].m == 0 && steps1d_smem(h) <= 200 * 1024;
+  return h.ndim == 1 && !h.elastic && h.dispersion != KWB_DISP_CHANGE && h.plan[0].m == 0 && steps1d_smem(h) <= 200 * 1024;
 }
 cudaError_t steps1d_prime(const SimDev &h) {
   return by_gaps(h.plan[0], [&](auto g) { return raise_dynamic_smem((const void *)k_steps_1d<decltype(g)::value>, steps1d_smem(h)); });

@@ -81,6 +81,8 @@ __host__ __device__ inline int line_slots(const FftPlan &p) { return fft_len(p) 
 enum { KWB_SLOT_LINE0 = 0, KWB_SLOT_LINE1 = 1, KWB_SLOT_LINE2 = 2, KWB_SLOT_EOS_FWD = 3, KWB_SLOT_EOS_INV = 4,
        KWB_SLOT_SPEC1 = 5, KWB_SLOT_SPEC2 = 6, KWB_SLOT_PLANE = 7, KWB_NSLOTS = 8 };
 
+// Dispersion: from the spectrum of the last step, or from that of the change since (dispersion_mode).
+enum { KWB_DISP_NONE = 0, KWB_DISP_LAST = 1, KWB_DISP_CHANGE = 2 };
 // Line-pass modes.
 enum { KWB_MODE_STEP = 0, KWB_MODE_INIT = 1 };
 // Spectrum-pass operations.
@@ -110,7 +112,9 @@ struct SimDev {
   float *u[3];
   float *rho[3];
   float2 *spec;
-  float2 *spec2;    // dispersion only: the spectrum of rho_eff at the last step, kept by the pass that multiplies
+  float2 *spec2;    // dispersion: the spectrum of rho_eff at the last step, kept by the pass that multiplies, or
+                    // (KWB_DISP_CHANGE) of its change since, from passes of its own
+  float *rho_prev;  // KWB_DISP_CHANGE: rho_eff at the last step
 
   const float *rho0;  // nullptr: scalar density
   const float *c0sq;  // nullptr: scalar sound speed
@@ -118,10 +122,10 @@ struct SimDev {
   const float *nlq;   // nullptr: scalar Q (nlq_s)
   float nlq_s;
   int nonlinear;
-  int dispersion;     // scalar c0 with :stokes absorption -> M2 and spec2
+  int dispersion;     // scalar c0 with :stokes absorption -> M2 and spec2 (KWB_DISP_*)
   int scalar_c;       // c^2 folded into M (scalar c0) vs applied per voxel
   const float *M;     // [Nz][Ny][n1]; plane pass: [n1][Nz][slot] or slot-major [n1][slot][z]
-  const float *M2;    // dispersion: multiplier of the last step's spectrum, [Nz][Ny][n1]
+  const float *M2;    // dispersion: multiplier of spec2, [Nz][Ny][n1]
 
   const float *pml_def[3];
   const float *pml_sg_def[3];
@@ -287,7 +291,7 @@ size_t line_pass_smem(const FftPlan &pl, int L);
 struct ElGrad;
 cudaError_t generic_prime(const SimDev &h);
 cudaError_t generic_line_pass(const SimDev &h, int axis, int mode, long long step_s, cudaStream_t st);
-cudaError_t generic_eos(const SimDev &h, bool fwd, long long step_s, cudaStream_t st);
+cudaError_t generic_eos(const SimDev &h, bool fwd, long long step_s, cudaStream_t st, bool change = false);
 cudaError_t generic_spec(const SimDev &h, int axis, int op, long long step_s, cudaStream_t st);
 cudaError_t generic_el_prime(const SimDev &h);
 cudaError_t generic_el_grad(const SimDev &h, int axis, const ElGrad &g, long long s, cudaStream_t st);
@@ -314,6 +318,10 @@ cudaError_t launch_spec_pass(const SimDev *d_sim, const SimDev &h, int axis, int
                              long long step_s, cudaStream_t st);
 cudaError_t launch_eos_x_inv(const SimDev *d_sim, const SimDev &h, long long step_s,
                              cudaStream_t st);
+// KWB_DISP_CHANGE: the spectrum of rho_eff's change since the last step, into spec2 (before the pass
+// that multiplies); `launches` of them
+cudaError_t launch_change_spectrum(const SimDev &h, long long step_s, cudaStream_t st);
+inline int change_launches(const SimDev &h) { return h.dispersion == KWB_DISP_CHANGE ? h.ndim : 0; }
 cudaError_t launch_tr_inject(const SimDev *d_sim, const SimDev &h, long long step_s,
                              cudaStream_t st);
 cudaError_t launch_sensor_gather(const SimDev *d_sim, const SimDev &h, const GroupDev *d_group,
@@ -490,7 +498,7 @@ cudaError_t build_pml_deficit(float *out, int N, int pml_size, double alpha, dou
 cudaError_t build_eos_multiplier(float *M, float *M2, const int N[3], const double d[3],
                                  double c_ref, double dt, double c_sq_fold, int absorbing,
                                  double tau, double eta, double y, const int *slot_ky,
-                                 const int *slot_kz, cudaStream_t st);
+                                 const int *slot_kz, int dispersion, cudaStream_t st);
 // Reorder a row-major grid array (NumPy order) into column-major (x fastest); ndim 2 or 3.
 cudaError_t transpose_to_column_major(double *out, const double *in, int ndim, const int N[3],
                                       cudaStream_t st);

@@ -125,6 +125,15 @@ cudaError_t launch_spec_pass(const SimDev *d_sim, const SimDev &h, int axis, int
   return generic_spec(h, axis, op, step_s, st);
 }
 
+cudaError_t launch_change_spectrum(const SimDev &h, long long step_s, cudaStream_t st) {
+  if (h.dispersion != KWB_DISP_CHANGE) return cudaSuccess;
+  SimDev c = h;  // on the in-place passes, with spec2 in the place of spec
+  c.spec = h.spec2;
+  cudaError_t e = generic_eos(c, true, step_s, st, true);
+  for (int a = 1; a < h.ndim && e == cudaSuccess; ++a) e = generic_spec(c, a, KWB_SPEC_FWD, step_s, st);
+  return e;
+}
+
 cudaError_t launch_tr_inject(const SimDev *d_sim, const SimDev &h, long long step_s,
                              cudaStream_t st) {
   if (h.n_tr <= 0) return cudaSuccess;

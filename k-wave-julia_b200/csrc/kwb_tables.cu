@@ -59,7 +59,7 @@ __global__ void k_build_pml_deficit(float *out, int N, int pml_size, double alph
 __global__ void k_build_eos_multiplier(float *M, float *M2, int Nx, int Ny, int Nz, double dx,
                                        double dy, double dz, double c_ref, double dt,
                                        double c_sq_fold, int absorbing, double tau, double eta,
-                                       double y, const int *slot_ky, const int *slot_kz) {
+                                       double y, const int *slot_ky, const int *slot_kz, int dispersion) {
   const int n1 = Nx / 2 + 1;
   const long long total = (long long)n1 * Ny * Nz;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -90,10 +90,12 @@ __global__ void k_build_eos_multiplier(float *M, float *M2, int Nx, int Ny, int 
   // Dispersion (first_order_steps.jl:255-263): M F - M2 (F - F_prev)/dt with F, F_prev the spectra of
   // rho_eff at this step and the last. The transform being linear, F_prev is the last step's
   // spectrum itself, kept by the pass that multiplies: M then holds M - M2/dt, and M2 holds M2/dt.
+  // With KWB_DISP_CHANGE the pass has the spectrum of the change instead: M, and -M2/dt.
   if (M2) {
     const double m2 = c_sq_fold * kappa * (eta * pow(kmag, y - 1.0)) * inv_total / dt;
-    M[idx] = (float)(m * inv_total - m2);
-    M2[idx] = (float)m2;
+    const bool change = dispersion == KWB_DISP_CHANGE;
+    M[idx] = (float)(change ? m * inv_total : m * inv_total - m2);
+    M2[idx] = (float)(change ? -m2 : m2);
   } else {
     M[idx] = (float)(m * inv_total);
   }
@@ -190,11 +192,11 @@ cudaError_t build_pml_deficit(float *out, int N, int pml_size, double alpha, dou
 cudaError_t build_eos_multiplier(float *M, float *M2, const int N[3], const double d[3],
                                  double c_ref, double dt, double c_sq_fold, int absorbing,
                                  double tau, double eta, double y, const int *slot_ky,
-                                 const int *slot_kz, cudaStream_t st) {
+                                 const int *slot_kz, int dispersion, cudaStream_t st) {
   const long long total = (long long)(N[0] / 2 + 1) * N[1] * N[2];
   k_build_eos_multiplier<<<blocks(total, 256), 256, 0, st>>>(M, M2, N[0], N[1], N[2], d[0],
                                                              d[1], d[2], c_ref, dt, c_sq_fold,
-                                                             absorbing, tau, eta, y, slot_ky, slot_kz);
+                                                             absorbing, tau, eta, y, slot_ky, slot_kz, dispersion);
   return cudaGetLastError();
 }
 cudaError_t transpose_to_column_major(double *out, const double *in, int ndim, const int N[3],

@@ -251,6 +251,7 @@ cudaError_t tune_schedule(SimDev &h, SimDev *d_scratch, cudaStream_t st, int pic
     for (int a : {1, 2, 0})
       if (a < D && (e = launch_line_pass(d, t, a, KWB_MODE_STEP, 0, st)) != cudaSuccess) return e;
     if (!t.fuse_xeos && (e = launch_eos_x_fwd(d, t, 0, st)) != cudaSuccess) return e;
+    if ((e = launch_change_spectrum(t, 0, st)) != cudaSuccess) return e;
     if (D == 2) {
       if ((e = launch_spec_pass(d, t, 1, KWB_SPEC_FWD_MUL_INV, 0, st)) != cudaSuccess) return e;
     } else if (D == 3 && t.plane) {

@@ -8,7 +8,7 @@ import threading
 import numpy as np
 import pytest
 
-from _util import assert_parity
+from _util import assert_parity, errors, run_gpu, run_oracle
 from test_gpu_any_length import TOL_L2, TOL_MAX, check, make_case
 
 pytestmark = pytest.mark.gpu
@@ -229,3 +229,23 @@ def test_tables_of_a_long_prime_side_do_not_dominate_its_set_up():
             ms[n] = min(ms[n], 1e3 * (time.perf_counter() - t))
             sim.close()
     assert ms[2039] < 4 * ms[2048], ms
+
+
+# the dispersion term at half and at four times the equation of state's own (its multiplier grows as
+# k^(y-1) / dt, and with tan(pi y/2) near y = 1), on grids fine enough and with steps short enough for the
+# scheme itself to be stable; also a step at a time, nonlinear, and with a Bluestein side.  Tolerance: the error
+# of the FP32 oracle, whose dispersion term transforms the change of the density, half as much again.
+@pytest.mark.parametrize("shape", [(512,), (60, 45), (64, 96), (34, 40), (20, 22, 18)])
+@pytest.mark.parametrize("dx,cfl,y,nonlinear", [(1e-4, 0.3, 1.02, False), (1e-5, 0.1, 1.5, False), (1e-5, 0.1, 1.5, True)])
+def test_strong_dispersion(shape, dx, cfl, y, nonlinear):
+    if len(shape) == 3 and y == 1.02:
+        dx, cfl = 2e-4, 0.2
+    l2 = {}
+    for seed in (11, 12, 13):
+        case = make_case(shape, seed=seed, stokes=True, source="p0", steps=120, record=("p_final",), nonlinear=nonlinear)
+        case.medium["alpha_power"] = y
+        case.d, case.dt = (dx,) * len(shape), cfl * dx / 1500.0
+        ref = run_oracle(case)
+        for name, out in (("gpu", run_gpu(case)), ("fp32", run_oracle(case, dtype=np.float32))):
+            l2[name] = l2.get(name, 0.0) + errors(out["p_final"], ref["p_final"])[0]
+    assert l2["gpu"] < 1.5 * l2["fp32"], l2
