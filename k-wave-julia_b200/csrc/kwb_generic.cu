@@ -676,7 +676,10 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
   const Lines<GAPS> &ln = sm.ln;
   float *P = const_cast<float *>(reinterpret_cast<const float *>(ln.tw + N + (N + 3) / 4));
   float *U = P + N, *Rh = U + N;
-  float2 *Prev = reinterpret_cast<float2 *>(P) + (3 * N + 1) / 2;  // dispersion: the last step's spectrum
+  // dispersion: the last step's spectrum, or this step's of the change since and the last rho_eff
+  float2 *Prev = reinterpret_cast<float2 *>(P) + (3 * N + 1) / 2;
+  float *Rp = reinterpret_cast<float *>(Prev + N);
+  const bool change = S.dispersion == KWB_DISP_CHANGE;
   const float *__restrict__ rho0 = S.rho0;
   auto set = [&](int i, float v) { ln.at(0, i) = make_float2(v, 0.f); };
   __syncthreads();  // the positions
@@ -684,7 +687,9 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     P[i] = S.p[i];
     U[i] = S.u[0][i];
     Rh[i] = S.rho[0][i];
-    if (S.dispersion) {  // spec2 holds k <= N/2; the field is real
+    if (change) {
+      Rp[i] = S.rho_prev[i];
+    } else if (S.dispersion) {  // spec2 holds k <= N/2; the field is real
       const float2 a = S.spec2[2 * i <= N ? i : N - i];
       Prev[sm.at_k[i]] = 2 * i <= N ? a : make_float2(a.x, -a.y);
     }
@@ -739,17 +744,24 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
       float f = Rh[i];
       if (S.nonlinear) f = f * fmaf(S.nlq ? __ldg(S.nlq + i) : S.nlq_s, f, 1.0f);
       if (S.c0sq) f = __ldg(S.c0sq + i) * f;
-      set(i, f);
+      set(i, change ? f - Rp[i] : f);
+      if (change) Rp[i] = f;
     }
     if (!S.dispersion) {
       conv_lines(ln, pl, S.eos1d);
     } else {
       fwd_lines(ln, pl);
+      if (change) {
+        for (int k = threadIdx.x; k < N; k += blockDim.x) Prev[k] = ln.at(0, k);
+        __syncthreads();
+        for (int i = threadIdx.x; i < N; i += blockDim.x) set(i, Rp[i]);
+        fwd_lines(ln, pl);
+      }
       for (int k = threadIdx.x; k < N; k += blockDim.x) {  // as k_spec_pass
         const int pos = sm.at_k[k], kk = 2 * k <= N ? k : N - k;
         const float m = __ldg(S.M + kk), m2 = __ldg(S.M2 + kk);
         const float2 z = ln.at(0, pos), b = Prev[pos];
-        Prev[pos] = z;
+        if (!change) Prev[pos] = z;
         ln.at(0, pos) = make_float2(fmaf(m2, b.x, m * z.x), fmaf(m2, b.y, m * z.y));
       }
       inv_lines(ln, pl);
@@ -770,7 +782,8 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
     S.p[i] = P[i];
     S.u[0][i] = U[i];
     S.rho[0][i] = Rh[i];
-    if (S.dispersion && 2 * i <= N) S.spec2[i] = Prev[sm.at_k[i]];
+    if (change) S.rho_prev[i] = Rp[i];
+    else if (S.dispersion && 2 * i <= N) S.spec2[i] = Prev[sm.at_k[i]];
   }
 }
 
@@ -787,7 +800,9 @@ size_t spectrum_pass_smem(const FftPlan &pl, int L) {
 }
 size_t steps1d_smem(const SimDev &h) {
   const int N = h.N[0];
-  return ((size_t)line_slots(h.plan[0]) * lines_pitch(1) + N + (N + 3) / 4 + (3 * N + 1) / 2 + (h.dispersion ? N : 0)) * sizeof(float2);
+  return ((size_t)line_slots(h.plan[0]) * lines_pitch(1) + N + (N + 3) / 4 + (3 * N + 1) / 2 + (h.dispersion ? N : 0) +
+          (h.dispersion == KWB_DISP_CHANGE ? (N + 1) / 2 : 0)) *
+         sizeof(float2);
 }
 
 }  // namespace
@@ -916,7 +931,7 @@ cudaError_t generic_el_grad(const SimDev &h, int axis, const ElGrad &g, long lon
   return cudaGetLastError();
 }
 bool steps1d_fits(const SimDev &h) {
-  return h.ndim == 1 && !h.elastic && h.dispersion != KWB_DISP_CHANGE && h.plan[0].m == 0 && steps1d_smem(h) <= 200 * 1024;
+  return h.ndim == 1 && !h.elastic && h.plan[0].m == 0 && steps1d_smem(h) <= 200 * 1024;
 }
 cudaError_t steps1d_prime(const SimDev &h) {
   return by_gaps(h.plan[0], [&](auto g) { return raise_dynamic_smem((const void *)k_steps_1d<decltype(g)::value>, steps1d_smem(h)); });

@@ -249,3 +249,19 @@ def test_strong_dispersion(shape, dx, cfl, y, nonlinear):
         for name, out in (("gpu", run_gpu(case)), ("fp32", run_oracle(case, dtype=np.float32))):
             l2[name] = l2.get(name, 0.0) + errors(out["p_final"], ref["p_final"])[0]
     assert l2["gpu"] < 1.5 * l2["fp32"], l2
+
+
+@pytest.mark.parametrize("n", [96, 1024, 2401, 34])
+def test_strong_dispersion_of_a_line_in_pieces(n):
+    """In one launch and pass by pass (profile), in turn; 34 points go pass by pass throughout."""
+    import kwave_b200 as kb
+    case = make_case((n,), source="p0", stokes=True, record=("p",), steps=90)
+    case.d, case.dt = (1e-5,), 1e-6 / 1500.0
+    g, m, s, sen, kw = case.to_api()
+    sim = kb.Simulation(g, m, s, sen, **kw)
+    assert sim.info()["launches_per_step"] == (5 if n == 34 else 1)
+    sim.advance(1)
+    sim.profile(5)
+    sim.advance(33)
+    assert_parity(sim.finish(), run_oracle(case), TOL_L2, TOL_MAX)
+    sim.close()
