@@ -1,4 +1,5 @@
-"""Edges of the accepted range: grids with one-point sides; reads of one simulation while another runs.
+"""Edges of the accepted range, and what stands beside the step: one-point sides, long lines, strong
+dispersion, source counts at a tile's limit, reads while another simulation runs, set-up costs, size rules.
 
 Tolerance as in test_gpu_any_length.py: about ten transforms a step, each adding some 2e-7 of relative
 rounding error, below 3e-5 over 60 steps.
@@ -265,3 +266,25 @@ def test_strong_dispersion_of_a_line_in_pieces(n):
     sim.advance(33)
     assert_parity(sim.finish(), run_oracle(case), TOL_L2, TOL_MAX)
     sim.close()
+
+
+# the register passes hold up to 96 source entries of a tile in shared memory, up to three a thread in the
+# narrowest, and read more in place: counts at that edge, all of them on the lines of one tile, which are at
+# least 8 consecutive rows (x) of 64 points or 4 columns (y) of 128
+@pytest.mark.parametrize("points", [32, 33, 95, 96, 97, 200])
+@pytest.mark.parametrize("tile", ["big", "mid", "small"])
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("source,mode", [("p", 0), ("u", 1)])
+def test_source_entries_at_the_edge_of_a_tile(points, tile, axis, source, mode, monkeypatch):
+    monkeypatch.setenv("KWB_TILE", tile)
+    shape = (64, 128)
+    case = make_case(shape, seed=points, source=source, points=1, mode=mode, steps=20)
+    rng = np.random.Generator(np.random.PCG64(points))
+    rows = np.zeros(shape, dtype=bool)  # the lines of a tile: rows y < 8 of the x pass, columns x < 4 of the y pass
+    rows[(slice(None), slice(0, 8)) if axis == 0 else (slice(0, 4), slice(None))] = True
+    mask = np.zeros(shape, dtype=bool)
+    mask.reshape(-1)[rng.choice(np.flatnonzero(rows), points, replace=False)] = True
+    sig = 1e5 * rng.standard_normal((points, 12))
+    case.source = dict(p_mask=mask, p=sig, p_mode=mode) if source == "p" else dict(
+        u_mask=mask, u_mode=mode, ux=1e-6 * sig, uy=-1e-6 * sig)
+    check(case)
