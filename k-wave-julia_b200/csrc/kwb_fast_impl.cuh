@@ -1600,7 +1600,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
 #pragma unroll
         for (int j = 0; j < B4; ++j) {
           const int idx = i0 + j;
-          if (valid && S.dispersion == KWB_DISP_LAST) S.spec2[mi[j]] = v[idx];
+          if (valid) S.spec2[mi[j]] = v[idx];
           v[idx] = pfma(pair(m2[j]), b[j], pmul(pair(m[idx]), v[idx]));
         }
       }

@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
       if (S.dispersion) {  // the spectrum of the step before (build_eos_multiplier)
         const float m2 = S.M2[q * n1 + k];
         const float2 b = __ldcg(S.spec2 + q * n1 + k);
-        if (S.dispersion == KWB_DISP_LAST) S.spec2[q * n1 + k] = v;
+        S.spec2[q * n1 + k] = v;
         v = make_float2(fmaf(m2, b.x, m * v.x), fmaf(m2, b.y, m * v.y));
       } else {
         v = cscale(v, m);
@@ -587,7 +587,8 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
   }
   if (op == KWB_SPEC_FWD_MUL_INV) {
     // the equation of state: times M, and with dispersion plus M2 times the spectrum of the step
-    // before, which this pass keeps in spec2, or of the change since (build_eos_multiplier)
+    // before, which this pass keeps in spec2, or of the change since (build_eos_multiplier; what is kept
+    // then is overwritten by the next step's)
     elements<false>(
         L, N, dL, pl.div_n,
         [&](int j, int l, int k) {
@@ -602,7 +603,7 @@ __global__ void __launch_bounds__(KWB_PASS_THREADS_MAX, 3)
           const float2 w = blue ? __ldg(pl.chirp + k) : zero;
           if (blue) z = cmul(z, w);
           if (S.dispersion) {
-            if (l < cnt && S.dispersion == KWB_DISP_LAST) S.spec2[at(l, k)] = z;
+            if (l < cnt) S.spec2[at(l, k)] = z;
             z = make_float2(fmaf(m2[j], b[j].x, m[j] * z.x), fmaf(m2[j], b[j].y, m[j] * z.y));
           } else {
             z = cscale(z, m[j]);
