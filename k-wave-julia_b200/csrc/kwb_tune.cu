@@ -118,27 +118,17 @@ struct Tuner {
   // Average device time of one launch of `go` (a time step) with the descriptor t (FLT_MAX if it
   // failed).  Grids whose steps take tens of microseconds are timed as their simulation runs them,
   // from a replayed graph: launched one by one, a 512^2 step took the host's 20 us whatever its
-  // tiles, and the choice was left to noise (128^2: 15.0 or 18.2 us a step).  The graph holds 4
-  // steps, is replayed once as a warm-up and then for a quarter of a millisecond, at least once and
-  // at most 4 times: 9 to 21 steps a candidate, what the first simulation of a shape waits for.
+  // tiles, and the choice was left to noise (128^2: 15.0 or 18.2 us a step).  The graph holds 0.6 ms
+  // of steps, 4 to 16 of them (with 4 at 640^2 its first and last kernels, which overlap nothing,
+  // led to a schedule of 41 us where 16 give 38.7), and is replayed once as a warm-up and once or
+  // twice, for 0.4 ms, to be timed: 11 steps a candidate from 150 us a step up, 35 to 51 below 40 us.  The
+  // first simulation of a shape waits for all that.
   template <class F>
   float time(F go) {
     cudaError_t e = cudaMemcpyAsync(d_t, &t, sizeof(SimDev), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = t.elastic ? el_prime(t) : prime_attributes(t);
     if (e == cudaSuccess) e = go();
-    constexpr int kGraphSteps = 4;
-    const bool replay = t.nvox <= (4LL << 20);
-    cudaGraphExec_t ex = nullptr;
-    if (replay && e == cudaSuccess) {
-      cudaGraph_t g = nullptr;
-      e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-      for (int r = 0; r < kGraphSteps && e == cudaSuccess; ++r) e = go();
-      const cudaError_t e2 = cudaStreamEndCapture(st, &g);
-      if (e == cudaSuccess) e = e2;
-      if (e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
-      if (g) cudaGraphDestroy(g);
-    }
-    // `n` runs of `once` between two events: milliseconds
+    // `n` runs of `once` between two events: milliseconds a run
     auto span = [&](int n, auto once) -> float {
       float ms = 0.f;
       if (e == cudaSuccess) e = cudaEventRecord(e0, st);
@@ -146,18 +136,27 @@ struct Tuner {
       if (e == cudaSuccess) e = cudaEventRecord(e1, st);
       if (e == cudaSuccess) e = cudaEventSynchronize(e1);
       if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-      return ms;
+      return ms / (float)n;
     };
-    float ms;
-    if (ex) {
+    const bool replay = t.nvox <= (4LL << 20);
+    float ms = span(replay ? 2 : 3, go);
+    if (replay && e == cudaSuccess) {
+      const int steps = std::max(4, std::min(16, (int)std::ceil(0.6f / std::max(ms, 1e-3f))));
+      cudaGraphExec_t ex = nullptr;
+      cudaGraph_t g = nullptr;
+      e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+      for (int r = 0; r < steps && e == cudaSuccess; ++r) e = go();
+      const cudaError_t e2 = cudaStreamEndCapture(st, &g);
+      if (e == cudaSuccess) e = e2;
+      if (e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
+      if (g) cudaGraphDestroy(g);
       auto once = [&] { return cudaGraphLaunch(ex, st); };
       const float warm = span(1, once);
-      const int n = std::max(1, std::min(4, (int)std::ceil(0.25f / std::max(warm, 1e-3f))));
-      ms = span(n, once) / (float)(n * kGraphSteps);
-      cudaStreamSynchronize(st);
-      cudaGraphExecDestroy(ex);
-    } else {
-      ms = span(3, go) / 3.f;
+      ms = span(warm < 0.4f ? 2 : 1, once) / (float)steps;
+      if (ex) {
+        cudaStreamSynchronize(st);
+        cudaGraphExecDestroy(ex);
+      }
     }
     if (e != cudaSuccess) {
       cudaGetLastError();

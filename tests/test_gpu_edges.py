@@ -189,7 +189,7 @@ def test_the_size_rule_of_a_small_grid_is_near_its_measured_schedule(monkeypatch
 
 
 def test_the_first_simulation_of_a_shape_waits_for_few_steps(monkeypatch):
-    """What measuring the schedule of a shape costs, in time steps of it: 24 candidates of 9 steps each at
+    """What measuring the schedule of a shape costs, in time steps of it: 24 candidates of 11 steps each at
     100 x 98 x 96 elastic, and the capture of their graphs.  With 33 steps a candidate it was 1000."""
     import time
     for k in ("KWB_TUNE", "KWB_TUNE_PICK", "KWB_TUNE_ORDER", "KWB_TILE"):
@@ -212,7 +212,7 @@ def test_the_first_simulation_of_a_shape_waits_for_few_steps(monkeypatch):
     sim.advance(32)
     step = min(sim.advance_timed(32) for _ in range(4)) / 32 * 1e-3
     sim.close()
-    assert took[0] - min(took[1:]) < 500 * step, (took, step)
+    assert took[0] - min(took[1:]) < 600 * step, (took, step)
 
 
 def test_tables_of_a_long_prime_side_do_not_dominate_its_set_up():
