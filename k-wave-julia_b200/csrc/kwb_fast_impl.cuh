@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(LT * F::G, MINB)
   // staggered deficits, then plain
   const float *pml_s = reinterpret_cast<const float *>(PML_S ? gn2 + E * RP : S.img[axis] + image_pairs<F>());
   // Contiguous tiles are 2L whole consecutive rows, so each field's tile is one block of
-  // memory: one bulk (TMA) copy per field.  Strided tiles (2L columns of N rows) are boxes of
+  // memory: one bulk (TMA) copy per field, or one a row where rows are padded apart.  Strided tiles (2L columns of N rows) are boxes of
   // the field's tensor map: N / tile_box_rows tiled TMA copies per field.  Each field's copies
   // complete on its own mbarrier (0 p, 1 rho0, 2 u_d, 3 rho_d; each used for one phase).
   // Tiled copies need 16-byte box rows and x offsets (2L a multiple of 4) and 128-byte aligned
