@@ -1026,7 +1026,7 @@ static void sched_store_locked(const std::string &key, const std::string &val) {
 }
 
 // Raised when the step kernels change, so that a file's measurements of older ones are not used.
-#define KWB_SCHED_GEN 5
+#define KWB_SCHED_GEN 6
 
 static std::string sched_key(int device, const SimDev &h) {
   // the device's name, asked once: the query takes 2.5 ms, a sixth of a 128^2 solve of 689 steps

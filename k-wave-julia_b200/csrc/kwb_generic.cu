@@ -843,14 +843,17 @@ cudaError_t generic_prime(const SimDev &h) {
     });
   return e;
 }
-// ... of a fluid pass: where it has at most two tiles an SM and the simulation runs alone, at least a
-// thread for every 4 elements, since its sweeps are then rounds of memory latency (us a step without a
-// measured schedule: 112^2 61 -> 52, 30 x 64 37.8 -> 32.4, 270 x 256 63.7 -> 45.9, 810 x 450 75 -> 71);
-// in larger grids, which hide it, more threads leave room for fewer CTAs (120 x 108 x 100 128 -> 141).
+// ... of a fluid pass: at least a thread for every 8 elements (first stages of radix 16 or 12 gave them 16
+// or 12: 112^2 in full-width tiles, as in a batch, 82 -> 64 us a step, 360 x 240 88 -> 71, 100^3 122 -> 108),
+// and where it has at most two tiles an SM and the simulation runs alone, for every 4, since its sweeps are
+// then rounds of memory latency (us a step without a measured schedule: 112^2 61 -> 52, 30 x 64 37.8 -> 32.4,
+// 270 x 256 63.7 -> 45.9, 810 x 450 75 -> 71); in larger grids, which hide it, so many threads leave room for
+// fewer CTAs (120 x 108 x 100: 8 elements 125, 4 141).
 static int fluid_threads(const SimDev &h, int axis, int L, int grid, int tuned) {
   const int thr = pass_threads(h.plan[axis], L, tuned);
-  if (tuned > 0 || !h.grid_fill || grid > 2 * h.num_sms) return thr;
-  return std::max(thr, std::min(KWB_PASS_THREADS_MAX, (L * h.plan[axis].n / 4 + 31) / 32 * 32));
+  if (tuned > 0) return thr;
+  const int each = h.grid_fill && grid <= 2 * h.num_sms ? 4 : 8;
+  return std::max(thr, std::min(KWB_PASS_THREADS_MAX, (L * h.plan[axis].n / each + 31) / 32 * 32));
 }
 cudaError_t generic_line_pass(const SimDev &h, int axis, int mode, long long step_s, cudaStream_t st) {
   const int L = h.L_line[axis];
