@@ -58,11 +58,11 @@ struct FftPlan {
   int nstages;
   int radix[KWB_MAX_STAGES];
   int m;
+  int sk;  // position pos of a line in shared memory is slot pos + (pos >> sk) (slots of line_slots)
   const float2 *chirp;
   const float2 *chirp_ft;
   const unsigned short *posof;  // digit-reversed position of each frequency (nullptr: worked out)
   FastDiv div_n;  // division by n
-  int sk;         // position pos of a line in shared memory is slot pos + (pos >> sk) (slots of line_slots)
   // per stage: butterflies per line, positions between a butterfly's elements, twiddle-table step,
   // and the divisions by the stride and by the radix
   int nbf[KWB_MAX_STAGES];
@@ -114,7 +114,6 @@ struct SimDev {
   float2 *spec;
   float2 *spec2;    // dispersion: the spectrum of rho_eff at the last step, kept by the pass that multiplies, or
                     // (KWB_DISP_CHANGE) of its change since, from passes of its own
-  float *rho_prev;  // KWB_DISP_CHANGE: rho_eff at the last step
 
   const float *rho0;  // nullptr: scalar density
   const float *c0sq;  // nullptr: scalar sound speed
@@ -229,6 +228,7 @@ struct SimDev {
   // for the launch that uses them (fast_line_pass); tile_tma_s = 0 stages by 16-byte cp.async.
   int tile_tma_s;
   int tile_box_rows;
+  float *rho_prev;  // KWB_DISP_CHANGE: rho_eff at the last step
   alignas(64) CUtensorMap tile_map[4];
 };
 
